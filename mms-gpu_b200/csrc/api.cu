@@ -417,7 +417,7 @@ int mms_ctx_create(const mms_grid *grid, const mms_params *params, const mms_sol
         if (ctx->s.kind == MMS_SOLVER_FMM || ctx->s.kind == MMS_SOLVER_SURROGATE) {
             if ((st = fmm_plan_create(ctx))) break;
         } else if (ctx->s.kind == MMS_SOLVER_DIRECT) {
-            if ((st = direct_build_table(ctx))) break;
+            if ((st = direct_prepare(ctx))) break;
         } else {
             mms_set_error("unknown solver kind %d", ctx->s.kind);
             st = MMS_ERR_ARG;
@@ -447,6 +447,7 @@ int mms_ctx_destroy(mms_ctx *ctx)
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     drop_graph(ctx);
     fmm_plan_destroy(ctx);
+    conv_plan_destroy(ctx->conv);
     void *bufs[] = {ctx->rho, ctx->phi, ctx->phibak, ctx->vecA, ctx->vecB, ctx->gtab, ctx->mat, ctx->M, ctx->A,
                     ctx->B, ctx->K, ctx->Mbak, ctx->Mfull, ctx->tstate, ctx->hext, ctx->stat_part, ctx->stats};
     for (void *b : bufs)
@@ -483,7 +484,7 @@ int mms_ctx_set_solver(mms_ctx *ctx, const mms_solver *solver)
     if (ctx->s.kind == MMS_SOLVER_FMM || ctx->s.kind == MMS_SOLVER_SURROGATE) {
         MMS_TRY(fmm_plan_create(ctx));
     } else if (ctx->s.kind == MMS_SOLVER_DIRECT) {
-        if (!ctx->gtab) MMS_TRY(direct_build_table(ctx));
+        MMS_TRY(direct_prepare(ctx));
     } else {
         mms_set_error("unknown solver kind %d", ctx->s.kind);
         return MMS_ERR_ARG;

@@ -1,0 +1,293 @@
+// Host side of the convolution (conv.cuh): plans, tables, and the launches of
+// the exact potential that keep the column store in device memory.
+#include <math.h>
+
+#include <algorithm>
+
+#include "conv.cuh"
+
+using namespace mmsconv;
+
+namespace {
+
+constexpr int ROW_PAIRS = 4;              // row pairs per CTA at most (a 128-byte run of a column each)
+constexpr size_t SMEM_MAX = 200 * 1024;   // per CTA
+constexpr int MAX_THREADS = 512;          // threads of a row or column CTA
+
+// tw[k] = exp(-2 pi i k / n)
+__global__ void k_conv_twiddle(double2 *__restrict__ tw, int n)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    double s, c;
+    sincospi(2.0 * k / n, &s, &c);
+    tw[k] = make_double2(c, -s);
+}
+
+// The even kernel's cosine transform along x, then along y: CTA = one (dz, y)
+// row into T[dz][kx][y], then one (kx, dz) column into G.  Offsets beyond
+// n / 2 are the mirror images of those below (weight 2; 0 and n / 2 are their
+// own); the largest offset of a grid is X - 1 < nx / 2 + 1.
+__global__ void k_conv_table_x(double *__restrict__ T, const double2 *__restrict__ tw, int n, int h, int hy, double dx,
+                               double dy, double dz)
+{
+    extern __shared__ double sg[];
+    const int y = blockIdx.x % hy, z = blockIdx.x / hy;
+    for (int x = threadIdx.x; x < h; x += blockDim.x) {
+        const double r2 = x * dx * (x * dx) + y * dy * (y * dy) + z * dz * (z * dz);
+        sg[x] = r2 == 0.0 ? 0.0 : dx * dy * dz / sqrt(r2) * (x == 0 || 2 * x == n ? 1.0 : 2.0);
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < h; k += blockDim.x) {
+        double s = 0.0;
+        int a = 0;  // k x mod n
+        for (int x = 0; x < h; x++) {
+            s = fma(sg[x], tw[a].x, s);
+            a += k;
+            if (a >= n) a -= n;
+        }
+        T[((long long)z * h + k) * hy + y] = s;
+    }
+}
+
+__global__ void k_conv_table_y(const double *__restrict__ T, double *__restrict__ G, const double2 *__restrict__ tw,
+                               int n, int h, int hx, int Z, double scale)
+{
+    extern __shared__ double sg[];
+    const int z = blockIdx.x % Z, kx = blockIdx.x / Z;
+    for (int y = threadIdx.x; y < h; y += blockDim.x)
+        sg[y] = T[((long long)z * hx + kx) * h + y] * (y == 0 || 2 * y == n ? 1.0 : 2.0);
+    __syncthreads();
+    for (int k = threadIdx.x; k < h; k += blockDim.x) {
+        double s = 0.0;
+        int a = 0;
+        for (int y = 0; y < h; y++) {
+            s = fma(sg[y], tw[a].x, s);
+            a += k;
+            if (a >= n) a -= n;
+        }
+        G[((long long)kx * Z + z) * h + k] = s * scale;
+    }
+}
+
+// ---- the passes with the columns in device memory [kx][z][y] -------------------
+// Three launches a potential.  Up to about 200 cells a side they are bound by
+// launch and barrier latency (4 us each), beyond by the column store's traffic
+// through L2 (32 bytes a cell and pass) and the FP64 passes.  Measured, whole
+// potential, against the pair sum: 64 x 64 x 3 13 us (100 us), 256 x 256 x 3
+// 22 us (2,056 us), 512 x 512 x 3 81 us (23.9 ms), 1024 x 1024 x 3 327 us
+// (382 ms); rel-L2 against the FP64 sum 2.5e-8 at every size, the rounding of
+// phi to FP32 (the compensated FP32 pair sum: 2e-7 .. 9e-7).  Columns are kept
+// [kx][z][y]: the column pass streams 16 Y bytes, and the four row pairs of a
+// row CTA write and read whole 128-byte lines of each column.
+struct RhoSrc {
+    const float *rho;
+    int X, Y;
+    __device__ __forceinline__ auto operator()(int z, int y) const
+    {
+        const float *r = rho + ((long long)z * Y + y) * X;
+        return [=](int x) { return r[x]; };
+    }
+};
+
+template <class PL, class SRC>
+__global__ void __launch_bounds__(MAX_THREADS) k_conv_rows(ConvDev c, SRC src, double2 *__restrict__ store)
+{
+    extern __shared__ __align__(16) double2 cbuf[];
+    pdl_begin();
+    const int np = c.Z * ((c.Y + 1) >> 1), p0 = blockIdx.x * c.fb, cs = c.cs;
+    rows_forward(PL{}, c, cbuf, p0, min(c.fb, np - p0), src, [=](int k) { return store + (long long)k * cs; });
+}
+
+template <class PL>
+__global__ void __launch_bounds__(MAX_THREADS) k_conv_columns(ConvDev c, double2 *__restrict__ store)
+{
+    extern __shared__ __align__(16) double2 cbuf[];
+    pdl_begin();
+    const int k0 = blockIdx.x * c.cpg, cs = c.cs;
+    columns(PL{}, c, cbuf, min(c.cpg, c.hx - k0), [=](int j) { return store + (long long)(k0 + j) * cs; },
+            [=](int j) { return k0 + j; });
+}
+
+template <class PL>
+__global__ void __launch_bounds__(MAX_THREADS) k_conv_back(ConvDev c, const double2 *__restrict__ store,
+                                                           float *__restrict__ phi)
+{
+    extern __shared__ __align__(16) double2 cbuf[];
+    pdl_begin();
+    const int np = c.Z * ((c.Y + 1) >> 1), p0 = blockIdx.x * c.fb, cs = c.cs, X = c.X, Y = c.Y;
+    rows_back(PL{}, c, cbuf, p0, min(c.fb, np - p0), [=](int k) { return store + (long long)k * cs; },
+              [=](int z, int y) {
+                  float *r = phi + ((long long)z * Y + y) * X;
+                  return [=](int x, float v) { r[x] = v; };
+              });
+}
+
+}  // namespace
+
+namespace mmsconv {
+
+// the shortest transform for m cells: at least 2 m - 1 long, so that no
+// wrap-around reaches a cell
+bool fft_plan(int m, int plans, FftPlan &p)
+{
+    for (int id = 0; id < plans; id++) {
+        with_plan(id, [&](auto pl) {
+            using PL = decltype(pl);
+            p = FftPlan{id, PL::n, PL::stride, PL::mmax};
+        });
+        if (p.n >= 2 * m - 1) return true;
+    }
+    return false;
+}
+
+// dims, plans and the layout of the column store; C > 0: in the shared memory
+// of a cluster of C CTAs of CT threads, C == 0: in device memory
+bool conv_layout(ConvDev &c, int X, int Y, int Z, int C)
+{
+    c = ConvDev{};
+    const int plans = C ? NSMALL : NPLANS;
+    if (X < 1 || Y < 1 || Z < 1 || Z > ZMAX || !fft_plan(X, plans, c.px) || !fft_plan(Y, plans, c.py)) return false;
+    c.X = X;
+    c.Y = Y;
+    c.Z = Z;
+    c.hx = c.px.n / 2 + 1;
+    c.hy = c.py.n / 2 + 1;
+    c.C = std::max(C, 1);
+    c.ncl = (c.hx + c.C - 1) / c.C;
+    c.ys = (Y + 1) / 2 * 2;
+    c.cs = Z * c.ys;
+    if (C) {
+        if (c.cs % 4 == 0) c.cs += 2;  // pairs of rows of neighbouring columns on different banks
+        const int pairs = (Z * (c.ys / 2) + C - 1) / C;
+        c.fb = std::min(pairs, CT / c.px.mmax);
+        c.cpg = std::max(1, std::min(c.ncl, CT / (c.py.mmax * Z)));
+    } else {
+        c.fb = std::max(1, std::min(ROW_PAIRS, MAX_THREADS / c.px.mmax));
+        c.cpg = 1;
+    }
+    return conv_smem(c, C) <= SMEM_MAX;
+}
+
+size_t conv_smem(const ConvDev &c, int C)
+{
+    const size_t rows = (size_t)c.fb * c.px.stride, cols = (size_t)c.cpg * c.Z * c.py.stride;
+    return ((C ? (size_t)c.ncl * c.cs : 0) + std::max(rows, cols)) * sizeof(double2);
+}
+
+size_t conv_table_bytes(const ConvDev &c)
+{
+    return ((size_t)c.px.n + c.py.n) * sizeof(double2) + (size_t)c.hx * c.hy * c.Z * sizeof(double);
+}
+
+// the twiddles and Ghat into `tab` (conv_table_bytes, 16-byte aligned); tmp:
+// hx hy Z doubles of scratch until the stream gets past the two launches
+int conv_build_tables(ConvDev &c, void *tab, double *tmp, double dx, double dy, double dz, cudaStream_t st,
+                      int64_t *launches)
+{
+    double2 *tx = (double2 *)tab, *ty = tx + c.px.n;
+    double *G = (double *)(ty + c.py.n);
+    k_conv_twiddle<<<div_up(c.px.n, 128), 128, 0, st>>>(tx, c.px.n);
+    k_conv_twiddle<<<div_up(c.py.n, 128), 128, 0, st>>>(ty, c.py.n);
+    k_conv_table_x<<<c.hy * c.Z, 128, c.hx * sizeof(double), st>>>(tmp, tx, c.px.n, c.hx, c.hy, dx, dy, dz);
+    k_conv_table_y<<<c.hx * c.Z, 128, c.hy * sizeof(double), st>>>(tmp, G, ty, c.py.n, c.hy, c.hx, c.Z,
+                                                                   0.5 / ((double)c.px.n * c.py.n));
+    MMS_CUDA_TRY(cudaGetLastError());
+    *launches += 4;
+    c.twx = tx;
+    c.twy = ty;
+    c.G = G;
+    return MMS_OK;
+}
+
+// raises a kernel's dynamic shared-memory limit (never lowers it: the limit is
+// shared by every context and ensemble)
+int conv_raise_smem(const void *kernel, size_t bytes)
+{
+    cudaFuncAttributes fa{};
+    MMS_CUDA_TRY(cudaFuncGetAttributes(&fa, kernel));
+    if ((size_t)fa.maxDynamicSharedSizeBytes < bytes)
+        MMS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return MMS_OK;
+}
+
+}  // namespace mmsconv
+
+struct ConvPlan {
+    ConvDev g{};               // columns in device memory
+    void *mem = nullptr;       // column store, then the tables
+    double2 *store = nullptr;
+    size_t bytes = 0;
+};
+
+// The convolution plan of a context's grid; *out stays NULL (and MMS_OK) where
+// the pair sum serves the grid: more than ZMAX layers, rows or columns beyond
+// the transforms' length, or no memory for the column store.
+int conv_plan_create(mms_ctx *ctx, ConvPlan **out)
+{
+    *out = nullptr;
+    ConvPlan pl;
+    if (!conv_layout(pl.g, ctx->g.xdim, ctx->g.ydim, ctx->g.zdim, 0)) return MMS_OK;
+    const size_t store = (size_t)pl.g.hx * pl.g.cs * sizeof(double2);
+    const size_t tmp = (size_t)pl.g.hx * pl.g.hy * pl.g.Z * sizeof(double);
+    const size_t first = (std::max(store, tmp) + 255) / 256 * 256;
+    pl.bytes = first + conv_table_bytes(pl.g);
+    if (cudaMalloc(&pl.mem, pl.bytes) != cudaSuccess) {
+        cudaGetLastError();  // not an error of the call: the pair sum needs no store
+        return MMS_OK;
+    }
+    pl.store = (double2 *)pl.mem;
+    int st = conv_build_tables(pl.g, (char *)pl.mem + first, (double *)pl.mem, ctx->g.dx, ctx->g.dy, ctx->g.dz,
+                               ctx->stream, &ctx->launches);
+    const size_t smem = conv_smem(pl.g, 0);
+    with_plan(pl.g.px.id, [&](auto p) {
+        if (!st) st = conv_raise_smem((const void *)k_conv_rows<decltype(p), RhoSrc>, smem);
+        if (!st) st = conv_raise_smem((const void *)k_conv_back<decltype(p)>, smem);
+    });
+    with_plan(pl.g.py.id, [&](auto p) {
+        if (!st) st = conv_raise_smem((const void *)k_conv_columns<decltype(p)>, smem);
+    });
+    if (st) {
+        cudaFree(pl.mem);
+        return st;
+    }
+    ctx->dev_bytes += pl.bytes;
+    *out = new ConvPlan(pl);
+    return MMS_OK;
+}
+
+void conv_plan_destroy(ConvPlan *pl)
+{
+    if (!pl) return;
+    cudaFree(pl->mem);
+    delete pl;
+}
+
+int launch_potential_conv(mms_ctx *ctx, ConvPlan *pl, const float *rho, float *phi)
+{
+    const ConvDev &c = pl->g;
+    const int pairs = c.Z * ((c.Y + 1) / 2);
+    const unsigned tr = (c.fb * c.px.mmax + 31) / 32 * 32;
+    const unsigned tc = std::min(MAX_THREADS, (c.Z * c.py.mmax + 31) / 32 * 32);
+    const size_t sr = (size_t)c.fb * c.px.stride * sizeof(double2);
+    const size_t sc = (size_t)c.cpg * c.Z * c.py.stride * sizeof(double2);
+    cudaError_t e = cudaSuccess;
+    with_plan(c.px.id, [&](auto p) {
+        e = launch_k(k_conv_rows<decltype(p), RhoSrc>, dim3(div_up(pairs, c.fb)), dim3(tr), sr, ctx->stream, c,
+                     RhoSrc{rho, c.X, c.Y}, pl->store);
+    });
+    MMS_CUDA_TRY(e);
+    MMS_LAUNCH_CHECK(ctx);
+    with_plan(c.py.id, [&](auto p) {
+        e = launch_k(k_conv_columns<decltype(p)>, dim3(div_up(c.hx, c.cpg)), dim3(tc), sc, ctx->stream, c, pl->store);
+    });
+    MMS_CUDA_TRY(e);
+    MMS_LAUNCH_CHECK(ctx);
+    with_plan(c.px.id, [&](auto p) {
+        e = launch_k(k_conv_back<decltype(p)>, dim3(div_up(pairs, c.fb)), dim3(tr), sr, ctx->stream, c,
+                     (const double2 *)pl->store, phi);
+    });
+    MMS_CUDA_TRY(e);
+    MMS_LAUNCH_CHECK(ctx);
+    return MMS_OK;
+}

@@ -101,7 +101,8 @@ constexpr int TIME_CTR = 3;
 //   [0] sum M.H  [1] max |MxH|  [2..4] sum M  [5] sum |M|  [6] count  [7] nonfinite flag
 constexpr int STAT_SLOTS = 8;
 
-struct FmmPlan;  // fmm.cu
+struct FmmPlan;   // fmm.cu
+struct ConvPlan;  // conv.cu
 
 struct mms_ctx {
     int device = 0;
@@ -118,7 +119,8 @@ struct mms_ctx {
     // device buffers
     float *rho = nullptr, *phi = nullptr;       // N
     float *vecA = nullptr, *vecB = nullptr;     // 3N FP32 AoS scratch (host API)
-    float *gtab = nullptr;                      // direct-sum kernel table X*Y*Z
+    ConvPlan *conv = nullptr;                   // exact potential as a convolution
+    float *gtab = nullptr;                      // pair-sum kernel table X*Y*Z, where there is no convolution plan
     uint8_t *mat = nullptr;                     // N
     double *M = nullptr, *A = nullptr, *B = nullptr, *K = nullptr;  // 3N each, SoA planes
     double *Mbak = nullptr;                     // 3N, controller backup
@@ -172,7 +174,11 @@ int launch_hfield_aos(mms_ctx *ctx, const float *M, const float *phi, double t, 
 int launch_rk4_stage(mms_ctx *ctx, int stage, const double *Mst, double *Mnext);
 int launch_stats(mms_ctx *ctx);
 
-int direct_build_table(mms_ctx *ctx);
+// exact potential: the convolution where the grid has a plan, else the pair sum
+int direct_prepare(mms_ctx *ctx);
+int conv_plan_create(mms_ctx *ctx, ConvPlan **out);
+void conv_plan_destroy(ConvPlan *pl);
+int launch_potential_conv(mms_ctx *ctx, ConvPlan *pl, const float *rho, float *phi);
 int launch_potential_direct(mms_ctx *ctx, const float *rho, float *phi);
 
 int fmm_plan_create(mms_ctx *ctx);
