@@ -475,7 +475,7 @@ def run_ours(args):
     ens = None
     if not args.no_ensemble:
         em = ensemble_measure(args, stream, flush, ws, rank)
-        ens = ensemble_summary(args, em, max_over_ranks(ws, em["ms_total"]), ws, fma_peak)
+        ens = ensemble_summary(args, em, max_over_ranks(ws, em["ms_total"]), ws)
 
     base = None
     if rank == 0 and not args.no_cpu_baseline:
@@ -756,7 +756,7 @@ def ensemble_measure(args, stream, flush, ws=1, rank=0):
     """The batched-ensemble configuration: `--ensemble-size` independent
     simulations (sides 16..64 in steps of 8, x3 layers, rectangle/disc/ellipse
     masks, random M, random in-plane |B| <= 50 mT; dt = 1e-13 s), one CUDA
-    graph per ensemble step, the direct kernel's shape autotuned first.  Under
+    graph per ensemble step.  Under
     torchrun the instances are partitioned over ranks by cost with no
     collective on the data path.  Returns the measurement (this rank's device
     time; the caller takes the max over ranks)."""
@@ -769,7 +769,7 @@ def ensemble_measure(args, stream, flush, ws=1, rank=0):
     ens = Ensemble([dims[i] for i in mine], (5e-9, 5e-9, 5e-9), mmsb200.make_params(external=True),
                    bext=[bext[i] for i in mine], stream=stream.cuda_stream)
     ens.state_set([masks[i] for i in mine], [Ms[i] for i in mine])
-    ew, q, direct_ms = ens.autotune(5)
+    _, _, potential_ms = ens.autotune(5)
     steps = max(args.steps, 20)
     ens.run_fixed(args.dt, max(args.warmup, 3), use_graph=True)
     ens.sync()
@@ -787,35 +787,25 @@ def ensemble_measure(args, stream, flush, ws=1, rank=0):
     cells = sum(int(np.prod(dims[i])) for i in mine)
     ens.close()
 
-    def charge_support(mask):
-        m = np.pad(mask != 0, 1)
-        sup = np.zeros_like(m)
-        for ax in range(3):
-            sup |= np.roll(m, 1, axis=ax) | np.roll(m, -1, axis=ax)
-        return int(sup[1:-1, 1:-1, 1:-1].sum())
-    # one FMA per (target, source) pair, sources = cells whose charge can be
-    # non-zero (a material neighbour), targets = all cells of the instance
-    pairs = float(sum(charge_support(masks[i]) * float(np.prod(dims[i])) for i in mine))
-    return {"steps": steps, "ms_total": ms_total, "cells": cells, "launches": int(launches), "pairs": pairs,
-            "direct_ms": direct_ms, "shape": {"warps": ew, "rows": q}, "instances": len(mine)}
+    return {"steps": steps, "ms_total": ms_total, "cells": cells, "launches": int(launches),
+            "potential_ms": potential_ms, "instances": len(mine)}
 
 
-def ensemble_summary(args, m, ms_total, ws, fma_peak):
+def ensemble_summary(args, m, ms_total, ws):
     value = m["steps"] / (ms_total * 1e-3)
-    achieved = 2 * m["pairs"] / (m["direct_ms"] * 1e-3) / 1e12
-    roof = {"kernel": "k_ens_direct (batched exact potential, persistent)", "bound": "fp32", "unit": "TFLOP/s",
-            "achieved": achieved, "peak": fma_peak, "frac": achieved / fma_peak,
-            "peak_source": "measured FP32 FMA microbenchmark (mms_diag_fma_tflops), of measured",
-            "algorithmic": "2 flops per target-source pair (sources: cells with a material neighbour; targets: "
-                           "all cells) of every instance, over the kernel's own mean time (CUDA events, "
-                           "back-to-back launches after autotuning)",
-            "kernel_ms": m["direct_ms"], "traffic": profile_traffic("k_ens_direct_512_instances")}
+    achieved = 28.0 * m["cells"] / (m["potential_ms"] * 1e-3) / 1e9
+    peak = hbm_peak()
+    roof = {"kernel": "k_ens_rows + k_ens_columns + k_ens_back (exact potential as a batched convolution)",
+            "bound": "hbm", "unit": "GB/s", "achieved": achieved, "peak": peak, "frac": achieved / peak,
+            "peak_source": "measured copy bandwidth, of measured",
+            "algorithmic": "the FP64 state read and phi written once: 28 bytes per cell of every instance, over the "
+                           "potential's own mean time (CUDA events, back-to-back evaluations)",
+            "kernel_ms": m["potential_ms"]}
     return {"metric": f"ensemble LLG RK4 steps/s ({args.ensemble_size} instances, 16..64 x 16..64 x 3)",
             "value": value, "unit": "ensemble steps/s", "steps": m["steps"], "ms_per_step": ms_total / m["steps"],
             "cells": m["cells"], "cell_steps_per_s": value * m["cells"], "gpu_launches": m["launches"],
-            "config": {"workload": "ensemble_rk4", "instances": args.ensemble_size, "solver": "direct (batched)",
-                       "dt_s": args.dt, "graph": "one CUDA graph per ensemble step",
-                       "autotuned_shape": m["shape"], "l2": "flushed between timed steps",
+            "config": {"workload": "ensemble_rk4", "instances": args.ensemble_size, "solver": "exact (batched)",
+                       "dt_s": args.dt, "graph": "one CUDA graph per ensemble step", "l2": "flushed between timed steps",
                        "parallelism": f"instance partition x{ws}" if ws > 1 else "single GPU"},
             "roofline": roof}
 
@@ -840,7 +830,7 @@ def run_ensemble(args):
         dist.destroy_process_group()
     if rank != 0:
         return 0
-    line = ensemble_summary(args, m, ms_total, ws, mmsb200.fma_tflops())
+    line = ensemble_summary(args, m, ms_total, ws)
     line.update({"n_gpus": ws, "warmup": max(args.warmup, 3), "higher_is_better": True, "scaling": "strong",
                  "vs_baseline": None, "dtype": "f32+f64", "data": "synthetic", "clocks": clk})
     print(json.dumps(line))

@@ -219,9 +219,9 @@ int mms_fmm_stage_times(mms_ctx *ctx, const float *rho, float *phi, int reps, do
 
 /* batched ensemble ----------------------------------------------------------- */
 /* Many independent simulations of uneven grid size (same cell size and
- * material) advance together: one kernel launch per RK4 stage for the whole
- * ensemble, driven by an instance offset table; exact direct-sum demag per
- * instance; one CUDA graph per step.  Each instance has its own constant
+ * material) advance together: a few kernel launches per RK4 stage for the whole
+ * ensemble, driven by an instance offset table; exact demag per instance; one
+ * CUDA graph per step.  Each instance has its own constant
  * external field bext (T), applied when params->external != 0.  No reference
  * counterpart (the reference runs one simulation per process). */
 typedef struct {
@@ -245,7 +245,10 @@ int mms_ens_run_fixed(mms_ens *ens, double dt, int nsteps, int use_graph);
 /* Chooses the batched direct kernel's shape by measurement on the current
  * state's charges: warps per CTA (4, 8, 16) x source rows staged per batch
  * (8, 16, 32), `reps` timed launches each; keeps the fastest (the results do
- * not depend on the shape).  Needs mms_ens_state_set first. */
+ * not depend on the shape).  Ensembles whose potential is evaluated as a
+ * convolution (every instance of at most 8 layers and 256 cells along y) have
+ * no shape to choose: *warps and *rows are those of the pair sum they do not
+ * run, *best_ms the time of one potential.  Needs mms_ens_state_set first. */
 int mms_ens_autotune(mms_ens *ens, int reps, int *warps, int *rows, double *best_ms);
 int mms_ens_sync(mms_ens *ens);
 

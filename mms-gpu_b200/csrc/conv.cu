@@ -10,8 +10,8 @@ using namespace mmsconv;
 
 namespace {
 
-constexpr int ROW_PAIRS = 4;              // row pairs per CTA at most (a 128-byte run of a column each)
 constexpr size_t SMEM_MAX = 200 * 1024;   // per CTA
+constexpr int ROW_PAIRS = 4;              // row pairs per CTA at most: small grids need the CTAs
 constexpr int MAX_THREADS = 512;          // threads of a row or column CTA
 
 // tw[k] = exp(-2 pi i k / n)
@@ -75,18 +75,19 @@ __global__ void k_conv_table_y(const double *__restrict__ T, double *__restrict_
 // launch and barrier latency (4 us each), beyond by the column store's traffic
 // through L2 (32 bytes a cell and pass) and the FP64 passes.  Measured, whole
 // potential, against the pair sum: 64 x 64 x 3 13 us (100 us), 256 x 256 x 3
-// 22 us (2,056 us), 512 x 512 x 3 81 us (23.9 ms), 1024 x 1024 x 3 327 us
+// 18.7 us (2,056 us), 512 x 512 x 3 68 us (23.9 ms), 1024 x 1024 x 3 294 us
 // (382 ms); rel-L2 against the FP64 sum 2.5e-8 at every size, the rounding of
 // phi to FP32 (the compensated FP32 pair sum: 2e-7 .. 9e-7).  Columns are kept
 // [kx][z][y]: the column pass streams 16 Y bytes, and the four row pairs of a
-// row CTA write and read whole 128-byte lines of each column.
+// row CTA write and read whole 128-byte lines of each column (the way back
+// with consecutive threads on consecutive pairs: 22 to 18.7 us at 256).
 struct RhoSrc {
     const float *rho;
     int X, Y;
     __device__ __forceinline__ auto operator()(int z, int y) const
     {
         const float *r = rho + ((long long)z * Y + y) * X;
-        return [=](int x) { return r[x]; };
+        return [=](int x, bool) { return r[x]; };
     }
 };
 
@@ -96,7 +97,7 @@ __global__ void __launch_bounds__(MAX_THREADS) k_conv_rows(ConvDev c, SRC src, d
     extern __shared__ __align__(16) double2 cbuf[];
     pdl_begin();
     const int np = c.Z * ((c.Y + 1) >> 1), p0 = blockIdx.x * c.fb, cs = c.cs;
-    rows_forward(PL{}, c, cbuf, p0, min(c.fb, np - p0), src, [=](int k) { return store + (long long)k * cs; });
+    rows_forward<row_pairs<PL>(MAX_THREADS, ROW_PAIRS)>(PL{}, c, cbuf, p0, min(c.fb, np - p0), src, [=](int k) { return store + (long long)k * cs; });
 }
 
 template <class PL>
@@ -116,7 +117,7 @@ __global__ void __launch_bounds__(MAX_THREADS) k_conv_back(ConvDev c, const doub
     extern __shared__ __align__(16) double2 cbuf[];
     pdl_begin();
     const int np = c.Z * ((c.Y + 1) >> 1), p0 = blockIdx.x * c.fb, cs = c.cs, X = c.X, Y = c.Y;
-    rows_back(PL{}, c, cbuf, p0, min(c.fb, np - p0), [=](int k) { return store + (long long)k * cs; },
+    rows_back<row_pairs<PL>(MAX_THREADS, ROW_PAIRS)>(PL{}, c, cbuf, p0, min(c.fb, np - p0), [=](int k) { return store + (long long)k * cs; },
               [=](int z, int y) {
                   float *r = phi + ((long long)z * Y + y) * X;
                   return [=](int x, float v) { r[x] = v; };
@@ -129,74 +130,62 @@ namespace mmsconv {
 
 // the shortest transform for m cells: at least 2 m - 1 long, so that no
 // wrap-around reaches a cell
-bool fft_plan(int m, int plans, FftPlan &p)
+static bool fft_plan(int m, int plans, int threads, int most, FftPlan &p, int *pairs)
 {
     for (int id = 0; id < plans; id++) {
         with_plan(id, [&](auto pl) {
             using PL = decltype(pl);
             p = FftPlan{id, PL::n, PL::stride, PL::mmax};
+            *pairs = row_pairs<PL>(threads, most);
         });
-        if (p.n >= 2 * m - 1) return true;
+        if (p.n >= 2 * m - 1 && p.mmax <= threads) return true;
     }
     return false;
 }
 
-// dims, plans and the layout of the column store; C > 0: in the shared memory
-// of a cluster of C CTAs of CT threads, C == 0: in device memory
-bool conv_layout(ConvDev &c, int X, int Y, int Z, int C)
+bool conv_layout(ConvDev &c, int X, int Y, int Z, int plans, int threads, int pairs, size_t *smem)
 {
     c = ConvDev{};
-    const int plans = C ? NSMALL : NPLANS;
-    if (X < 1 || Y < 1 || Z < 1 || Z > ZMAX || !fft_plan(X, plans, c.px) || !fft_plan(Y, plans, c.py)) return false;
+    int unused = 0;
+    if (X < 1 || Y < 1 || Z < 1 || Z > ZMAX || !fft_plan(X, plans, threads, pairs, c.px, &c.fb) ||
+        !fft_plan(Y, plans, threads, pairs, c.py, &unused))
+        return false;
     c.X = X;
     c.Y = Y;
     c.Z = Z;
     c.hx = c.px.n / 2 + 1;
     c.hy = c.py.n / 2 + 1;
-    c.C = std::max(C, 1);
-    c.ncl = (c.hx + c.C - 1) / c.C;
     c.ys = (Y + 1) / 2 * 2;
     c.cs = Z * c.ys;
-    if (C) {
-        if (c.cs % 4 == 0) c.cs += 2;  // pairs of rows of neighbouring columns on different banks
-        const int pairs = (Z * (c.ys / 2) + C - 1) / C;
-        c.fb = std::min(pairs, CT / c.px.mmax);
-        c.cpg = std::max(1, std::min(c.ncl, CT / (c.py.mmax * Z)));
-    } else {
-        c.fb = std::max(1, std::min(ROW_PAIRS, MAX_THREADS / c.px.mmax));
-        c.cpg = 1;
-    }
-    return conv_smem(c, C) <= SMEM_MAX;
-}
-
-size_t conv_smem(const ConvDev &c, int C)
-{
-    const size_t rows = (size_t)c.fb * c.px.stride, cols = (size_t)c.cpg * c.Z * c.py.stride;
-    return ((C ? (size_t)c.ncl * c.cs : 0) + std::max(rows, cols)) * sizeof(double2);
+    c.cpg = std::max(1, threads / (Z * c.py.mmax));
+    const size_t s = std::max((size_t)c.fb * c.px.stride, (size_t)c.cpg * Z * c.py.stride) * sizeof(double2);
+    *smem = s;
+    return s <= SMEM_MAX;
 }
 
 size_t conv_table_bytes(const ConvDev &c)
 {
-    return ((size_t)c.px.n + c.py.n) * sizeof(double2) + (size_t)c.hx * c.hy * c.Z * sizeof(double);
+    const size_t b = ((size_t)c.px.n + c.py.n) * sizeof(double2) + (size_t)c.hx * c.hy * c.Z * sizeof(double);
+    return (b + 255) / 256 * 256;
 }
 
-// the twiddles and Ghat into `tab` (conv_table_bytes, 16-byte aligned); tmp:
-// hx hy Z doubles of scratch until the stream gets past the two launches
-int conv_build_tables(ConvDev &c, void *tab, double *tmp, double dx, double dy, double dz, cudaStream_t st,
+size_t conv_table_scratch(const ConvDev &c) { return (size_t)c.hx * c.hy * c.Z * sizeof(double); }
+
+int conv_build_tables(ConvDev &c, void *tab, double *scratch, double dx, double dy, double dz, cudaStream_t st,
                       int64_t *launches)
 {
     double2 *tx = (double2 *)tab, *ty = tx + c.px.n;
-    double *G = (double *)(ty + c.py.n);
+    double *g = (double *)(ty + c.py.n);
     k_conv_twiddle<<<div_up(c.px.n, 128), 128, 0, st>>>(tx, c.px.n);
     k_conv_twiddle<<<div_up(c.py.n, 128), 128, 0, st>>>(ty, c.py.n);
-    k_conv_table_x<<<c.hy * c.Z, 128, c.hx * sizeof(double), st>>>(tmp, tx, c.px.n, c.hx, c.hy, dx, dy, dz);
-    k_conv_table_y<<<c.hx * c.Z, 128, c.hy * sizeof(double), st>>>(tmp, G, ty, c.py.n, c.hy, c.hx, c.Z,
+    k_conv_table_x<<<c.hy * c.Z, 128, c.hx * sizeof(double), st>>>(scratch, tx, c.px.n, c.hx, c.hy, dx, dy, dz);
+    k_conv_table_y<<<c.hx * c.Z, 128, c.hy * sizeof(double), st>>>(scratch, g, ty, c.py.n, c.hy, c.hx, c.Z,
                                                                    0.5 / ((double)c.px.n * c.py.n));
     MMS_CUDA_TRY(cudaGetLastError());
     *launches += 4;
     c.twx = tx;
     c.twy = ty;
-    c.G = G;
+    c.G = g;
     return MMS_OK;
 }
 
@@ -227,19 +216,20 @@ int conv_plan_create(mms_ctx *ctx, ConvPlan **out)
 {
     *out = nullptr;
     ConvPlan pl;
-    if (!conv_layout(pl.g, ctx->g.xdim, ctx->g.ydim, ctx->g.zdim, 0)) return MMS_OK;
-    const size_t store = (size_t)pl.g.hx * pl.g.cs * sizeof(double2);
-    const size_t tmp = (size_t)pl.g.hx * pl.g.hy * pl.g.Z * sizeof(double);
-    const size_t first = (std::max(store, tmp) + 255) / 256 * 256;
-    pl.bytes = first + conv_table_bytes(pl.g);
+    ConvDev &c = pl.g;
+    size_t smem = 0;
+    if (!conv_layout(c, ctx->g.xdim, ctx->g.ydim, ctx->g.zdim, NPLANS, MAX_THREADS, ROW_PAIRS, &smem)) return MMS_OK;
+    c.cpg = 1;  // a CTA per column: the launch has few enough
+    const size_t store = (size_t)c.hx * c.cs * sizeof(double2);
+    const size_t first = (std::max(store, conv_table_scratch(c)) + 255) / 256 * 256;
+    pl.bytes = first + conv_table_bytes(c);
     if (cudaMalloc(&pl.mem, pl.bytes) != cudaSuccess) {
         cudaGetLastError();  // not an error of the call: the pair sum needs no store
         return MMS_OK;
     }
     pl.store = (double2 *)pl.mem;
-    int st = conv_build_tables(pl.g, (char *)pl.mem + first, (double *)pl.mem, ctx->g.dx, ctx->g.dy, ctx->g.dz,
+    int st = conv_build_tables(c, (char *)pl.mem + first, (double *)pl.mem, ctx->g.dx, ctx->g.dy, ctx->g.dz,
                                ctx->stream, &ctx->launches);
-    const size_t smem = conv_smem(pl.g, 0);
     with_plan(pl.g.px.id, [&](auto p) {
         if (!st) st = conv_raise_smem((const void *)k_conv_rows<decltype(p), RhoSrc>, smem);
         if (!st) st = conv_raise_smem((const void *)k_conv_back<decltype(p)>, smem);

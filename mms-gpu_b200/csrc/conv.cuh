@@ -23,10 +23,9 @@
 // long as the butterflies).  The inverse is the forward transform with real
 // and imaginary parts exchanged before and after.
 //
-// The columns between the passes live either in the shared memory of a
-// cluster of CTAs (small grids and ensemble instances: one launch, the rows'
-// results stored to the owner of their column through distributed shared
-// memory) or in device memory (larger grids: a launch per pass).
+// This header is the form with the columns in device memory, a launch per
+// pass; conv_sim.cu keeps those of small grids in the shared memory of a
+// cluster of CTAs.
 #pragma once
 
 #include "mms_internal.cuh"
@@ -34,7 +33,6 @@
 namespace mmsconv {
 
 constexpr int ZMAX = 8;      // most layers of a column (held in registers)
-constexpr int CT = 256;      // threads of a cluster's CTAs
 
 // A transform of the product of the radices, the largest first: 16 only there,
 // where no twiddles are held beside its 16 elements.
@@ -47,39 +45,26 @@ struct Radices {
     // padded position of element i: i + (i >> shift) keeps the stores of the
     // first pass (R0 apart) on different banks
     static constexpr int shift = R0 == 16 ? 4 : R0 == 8 ? 3 : 2;
-    static constexpr int stride = n + (n >> shift) + 1;
+    static constexpr int stride = (n + (n >> shift)) | 1;  // odd: lanes on different transforms, different banks
 };
 
 constexpr int NPLANS = 19;
-// the lengths up to the SMALL-th are also those of the clusters' kernels
-constexpr int NSMALL = 11;
-
-#define MMS_CONV_SMALL_PLANS(f)                                 \
-    case 0: f(Radices<4, 4>{}); break;         /* 16 */          \
-    case 1: f(Radices<8, 4>{}); break;         /* 32 */          \
-    case 2: f(Radices<16, 3>{}); break;        /* 48 */          \
-    case 3: f(Radices<8, 8>{}); break;         /* 64 */          \
-    case 4: f(Radices<16, 5>{}); break;        /* 80 */          \
-    case 5: f(Radices<8, 4, 3>{}); break;      /* 96 */          \
-    case 6: f(Radices<16, 8>{}); break;        /* 128 */         \
-    case 7: f(Radices<8, 5, 4>{}); break;      /* 160 */         \
-    case 8: f(Radices<8, 8, 3>{}); break;      /* 192 */         \
-    case 9: f(Radices<8, 8, 4>{}); break;      /* 256 */         \
-    case 10: f(Radices<8, 8, 5>{}); break;     /* 320 */
-
-template <class F>
-__device__ __forceinline__ void with_small_plan(int id, F &&f)
-{
-    switch (id) {
-        MMS_CONV_SMALL_PLANS(f)
-    }
-}
 
 template <class F>
 void with_plan(int id, F &&f)
 {
     switch (id) {
-        MMS_CONV_SMALL_PLANS(f)
+    case 0: f(Radices<4, 4>{}); break;          // 16
+    case 1: f(Radices<8, 4>{}); break;          // 32
+    case 2: f(Radices<8, 6>{}); break;          // 48
+    case 3: f(Radices<8, 8>{}); break;          // 64
+    case 4: f(Radices<8, 10>{}); break;         // 80
+    case 5: f(Radices<8, 12>{}); break;       // 96
+    case 6: f(Radices<16, 8>{}); break;         // 128
+    case 7: f(Radices<16, 10>{}); break;       // 160
+    case 8: f(Radices<8, 8, 3>{}); break;       // 192
+    case 9: f(Radices<8, 8, 4>{}); break;       // 256
+    case 10: f(Radices<8, 8, 5>{}); break;      // 320
     case 11: f(Radices<16, 8, 3>{}); break;     // 384
     case 12: f(Radices<8, 8, 8>{}); break;      // 512
     case 13: f(Radices<16, 8, 5>{}); break;     // 640
@@ -91,17 +76,45 @@ void with_plan(int id, F &&f)
     }
 }
 
+// the lengths up to 512 in one kernel (the batched form: a CTA's length is its
+// instance's)
+constexpr int NBATCH = 13;
+template <class F>
+__device__ __forceinline__ void with_batch_plan(int id, F &&f)
+{
+    switch (id) {
+    case 0: f(Radices<4, 4>{}); break;
+    case 1: f(Radices<8, 4>{}); break;
+    case 2: f(Radices<8, 6>{}); break;
+    case 3: f(Radices<8, 8>{}); break;
+    case 4: f(Radices<8, 10>{}); break;
+    case 5: f(Radices<8, 12>{}); break;
+    case 6: f(Radices<16, 8>{}); break;
+    case 7: f(Radices<16, 10>{}); break;
+    case 8: f(Radices<8, 8, 3>{}); break;
+    case 9: f(Radices<8, 8, 4>{}); break;
+    case 10: f(Radices<8, 8, 5>{}); break;
+    case 11: f(Radices<16, 8, 3>{}); break;
+    case 12: f(Radices<8, 8, 8>{}); break;
+    }
+}
+
 struct FftPlan {
     int id, n, stride, mmax;
 };
 
-// One grid's convolution.  rank c of C owns the columns kx = c, c + C, ...
+// row pairs per CTA of `threads`, at most `most` (4: a 128-byte run of each column)
+template <class PL>
+__host__ __device__ constexpr int row_pairs(int threads, int most)
+{
+    return threads / PL::mmax < 1 ? 1 : threads / PL::mmax > most ? most : threads / PL::mmax;
+}
+
+// One grid's convolution with the column store in device memory
 struct ConvDev {
     int X, Y, Z, hx, hy;
-    int C, ncl;      // CTAs of the cluster, columns per CTA
     int ys, cs;      // elements between layers / columns in the column store
-    int fb, cpg;     // row pairs per group, columns per group
-    int pad;
+    int fb, cpg;     // row pairs and columns per CTA
     FftPlan px, py;
     const double2 *twx, *twy;  // exp(-2 pi i k / n), k < n
     const double *G;           // [kx < hx][|dz| < Z][ky < hy], scaled by 1 / (2 nx ny)
@@ -160,12 +173,55 @@ __host__ __device__ __forceinline__ void dft<5>(double2 *v)
     v[2] = m2 + s2;
     v[3] = m2 - s2;
 }
+// N1 N2, coprime: element N2 i1 + N1 i2 (mod n) to output k with k = k1 (mod
+// N1) and k = k2 (mod N2), no twiddles (Good 1958)
+template <int N1, int N2>
+__host__ __device__ __forceinline__ void dft_coprime(double2 *v)
+{
+    constexpr int n = N1 * N2;
+    double2 t[N2][N1];
+#pragma unroll
+    for (int i2 = 0; i2 < N2; i2++) {
+#pragma unroll
+        for (int i1 = 0; i1 < N1; i1++) t[i2][i1] = v[(N2 * i1 + N1 * i2) % n];
+        dft<N1>(t[i2]);
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < N1; k1++) {
+        double2 u[N2];
+#pragma unroll
+        for (int i2 = 0; i2 < N2; i2++) u[i2] = t[i2][k1];
+        dft<N2>(u);
+#pragma unroll
+        for (int k2 = 0; k2 < N2; k2++)
+#pragma unroll
+            for (int k = k1; k < n; k += N1)
+                if (k % N2 == k2) v[k] = u[k2];  // the output with these residues
+    }
+}
 template <>
-__host__ __device__ __forceinline__ void dft<8>(double2 *v)
+__host__ __device__ __forceinline__ void dft<2>(double2 *v)
+{
+    const double2 a = v[0], b = v[1];
+    v[0] = a + b;
+    v[1] = a - b;
+}
+template <>
+__host__ __device__ __forceinline__ void dft<6>(double2 *v) { dft_coprime<2, 3>(v); }
+template <>
+__host__ __device__ __forceinline__ void dft<10>(double2 *v) { dft_coprime<2, 5>(v); }
+template <>
+__host__ __device__ __forceinline__ void dft<12>(double2 *v) { dft_coprime<4, 3>(v); }
+
+// R = 4, 8, 16: what follows the sub-transforms of 4 over v[j], v[j + R/4], ...
+template <int R>
+__host__ __device__ __forceinline__ void dft_rest(double2 *v);
+template <>
+__host__ __device__ __forceinline__ void dft_rest<4>(double2 *) {}
+template <>
+__host__ __device__ __forceinline__ void dft_rest<8>(double2 *v)
 {
     constexpr double H = 0.70710678118654752440;
-    dft4(v[0], v[2], v[4], v[6]);
-    dft4(v[1], v[3], v[5], v[7]);
     const double2 o0 = v[1], o2 = mul_mi(v[5]);
     const double2 o1 = make_double2(H * (v[3].x + v[3].y), H * (v[3].y - v[3].x));
     const double2 o3 = make_double2(H * (v[7].y - v[7].x), -H * (v[7].x + v[7].y));
@@ -180,11 +236,9 @@ __host__ __device__ __forceinline__ void dft<8>(double2 *v)
     v[7] = e3 - o3;
 }
 template <>
-__host__ __device__ __forceinline__ void dft<16>(double2 *v)
+__host__ __device__ __forceinline__ void dft_rest<16>(double2 *v)
 {
     constexpr double H = 0.70710678118654752440, C = 0.92387953251128675613, S = 0.38268343236508977173;
-#pragma unroll
-    for (int j = 0; j < 4; j++) dft4(v[j], v[j + 4], v[j + 8], v[j + 12]);
     // v[j + 4 k] is output k of sub-transform j: times exp(-2 pi i j k / 16)
     v[5] = cmul(v[5], make_double2(C, -S));
     v[6] = make_double2(H * (v[6].x + v[6].y), H * (v[6].y - v[6].x));
@@ -208,51 +262,102 @@ __host__ __device__ __forceinline__ void dft<16>(double2 *v)
         }
 }
 
+template <>
+__host__ __device__ __forceinline__ void dft<8>(double2 *v)
+{
+    dft4(v[0], v[2], v[4], v[6]);
+    dft4(v[1], v[3], v[5], v[7]);
+    dft_rest<8>(v);
+}
+template <>
+__host__ __device__ __forceinline__ void dft<16>(double2 *v)
+{
+#pragma unroll
+    for (int j = 0; j < 4; j++) dft4(v[j], v[j + 4], v[j + 8], v[j + 12]);
+    dft_rest<16>(v);
+}
+
+// DFT of v with the upper half of its inputs zero (the padding of a first pass)
+template <int R>
+__host__ __device__ __forceinline__ void dft_padded(double2 *v)
+{
+    if constexpr (R == 4 || R == 8 || R == 16) {
+        constexpr int H = R / 4;  // sub-transforms of 4, of which two inputs are not zero
+#pragma unroll
+        for (int j = 0; j < H; j++) {
+            const double2 a = v[j], b = v[j + H], c = mul_mi(b);
+            v[j] = a + b;
+            v[j + H] = a + c;
+            v[j + 2 * H] = a - b;
+            v[j + 3 * H] = a - c;
+        }
+        dft_rest<R>(v);
+    } else {
+#pragma unroll
+        for (int q = R / 2; q < R; q++) v[q] = make_double2(0.0, 0.0);
+        dft<R>(v);
+    }
+}
+
 // host side (conv.cu)
-bool fft_plan(int m, int plans, FftPlan &p);
-bool conv_layout(ConvDev &c, int X, int Y, int Z, int C);
-size_t conv_smem(const ConvDev &c, int C);
+// dims, plans and layout of a grid for CTAs of `threads` (at most `pairs` row
+// pairs) and the first `plans` lengths; false where it has none.  *smem: what a row or column CTA needs.
+bool conv_layout(ConvDev &c, int X, int Y, int Z, int plans, int threads, int pairs, size_t *smem);
+// bytes of the twiddles and Ghat for these lengths and layers, and of the
+// scratch their construction needs
 size_t conv_table_bytes(const ConvDev &c);
-int conv_build_tables(ConvDev &c, void *tab, double *tmp, double dx, double dy, double dz, cudaStream_t st,
+size_t conv_table_scratch(const ConvDev &c);
+// builds them in `tab` (256-byte aligned); scratch is free once the stream is
+// past the launches
+int conv_build_tables(ConvDev &c, void *tab, double *scratch, double dx, double dy, double dz, cudaStream_t st,
                       int64_t *launches);
 int conv_raise_smem(const void *kernel, size_t bytes);
 
-// Pass number PASS of nf transforms, one butterfly per thread (nf n / R <=
+// One Stockham pass of nf transforms, one butterfly per thread (nf n / R <=
 // blockDim): ld(f) gives a reader of transform f's elements, st(f) a writer.
 // sync: between the reads and the writes (in-place passes; one with another
-// source or destination does without).
-template <class PL, int NS, int R, class LD, class ST>
+// source or destination does without).  LOW_IN: elements from n / 2 up are
+// padding and not read; LOW_OUT: those of the result are not wanted.  FB > 0:
+// consecutive threads take the same butterfly of FB consecutive transforms
+// (whose elements the source holds side by side), else consecutive ones of one.
+template <class PL, int NS, int R, bool LOW_IN, bool LOW_OUT, int FB, class LD, class ST>
 __device__ __forceinline__ void fft_pass(const double2 *__restrict__ tw, int nf, bool sync, LD ld, ST st)
 {
     constexpr int m = PL::n / R;
-    const int f = threadIdx.x / m, b = threadIdx.x % m;
-    const bool on = f < nf;
+    const int f = FB > 0 ? threadIdx.x % (FB > 0 ? FB : 1) : threadIdx.x / m;
+    const int b = FB > 0 ? threadIdx.x / (FB > 0 ? FB : 1) : threadIdx.x % m;
+    const bool on = f < nf && b < m;
     double2 v[R];
     const int k = b % NS, base = (b / NS) * NS * R + k;
     if (on) {
         const auto get = ld(f);
 #pragma unroll
-        for (int q = 0; q < R; q++) v[q] = get(b + q * m);
+        for (int q = 0; q < (LOW_IN ? R / 2 : R); q++) v[q] = get(b + q * m);
         if constexpr (NS > 1) {
             const int step = k * (m / NS);  // n / (NS R)
 #pragma unroll
             for (int q = 1; q < R; q++) v[q] = cmul(v[q], __ldg(&tw[q * step]));
         }
-        dft<R>(v);
+        if constexpr (LOW_IN)
+            dft_padded<R>(v);
+        else
+            dft<R>(v);
     }
     if (sync) __syncthreads();
     if (on) {
         const auto put = st(f);
 #pragma unroll
-        for (int q = 0; q < R; q++) put(base + q * NS, v[q]);
+        for (int q = 0; q < R; q++)
+            if (!LOW_OUT || 2 * q * NS < PL::n) put(base + q * NS, v[q]);
     }
 }
 
 // nf transforms of source ld into buf (TO_BUF) or st.  buf holds nf padded
 // transforms and is not in use when called, unless ld reads it (IN_PLACE:
 // element i of transform f at its own place); the caller synchronises
-// afterwards.
-template <bool TO_BUF, bool IN_PLACE, int R0, int R1, int R2, int R3, class LD, class ST>
+// afterwards.  A source other than buf has n / 2 elements at most, and so has
+// the result that goes to st.  FB: of the first pass.
+template <bool TO_BUF, bool IN_PLACE, int FB, int R0, int R1, int R2, int R3, class LD, class ST>
 __device__ __forceinline__ void fft_batch(Radices<R0, R1, R2, R3>, const double2 *tw, double2 *buf, int nf, LD ld, ST st)
 {
     using PL = Radices<R0, R1, R2, R3>;
@@ -264,48 +369,48 @@ __device__ __forceinline__ void fft_batch(Radices<R0, R1, R2, R3>, const double2
         double2 *p = buf + f * PL::stride;
         return [=](int i, double2 v) { p[i + (i >> PL::shift)] = v; };
     };
-    fft_pass<PL, 1, R0>(tw, nf, IN_PLACE, ld, bst);
+    fft_pass<PL, 1, R0, TO_BUF && !IN_PLACE, false, FB>(tw, nf, IN_PLACE, ld, bst);
     __syncthreads();
     if constexpr (R2 > 1) {
-        fft_pass<PL, R0, R1>(tw, nf, true, bld, bst);
+        fft_pass<PL, R0, R1, false, false, 0>(tw, nf, true, bld, bst);
         __syncthreads();
     }
     if constexpr (R3 > 1) {
-        fft_pass<PL, R0 * R1, R2>(tw, nf, true, bld, bst);
+        fft_pass<PL, R0 * R1, R2, false, false, 0>(tw, nf, true, bld, bst);
         __syncthreads();
     }
     if constexpr (TO_BUF)
-        fft_pass<PL, PL::n / PL::last, PL::last>(tw, nf, true, bld, bst);
+        fft_pass<PL, PL::n / PL::last, PL::last, false, false, 0>(tw, nf, true, bld, bst);
     else
-        fft_pass<PL, PL::n / PL::last, PL::last>(tw, nf, false, bld, st);
+        fft_pass<PL, PL::n / PL::last, PL::last, false, true, 0>(tw, nf, false, bld, st);
 }
 
-// Rows forward for pairs p0 .. p0 + np - 1 (np <= fb; pair p: layer p / hp,
+// Rows forward for pairs p0 .. p0 + np - 1 (np <= FB; pair p: layer p / hp,
 // rows y0 = 2 (p % hp) and y0 + 1): src(z, y) gives a reader of the charges of
-// a row, col(kx) the column store of kx.  buf is free on return.
-template <class PL, class SRC, class COL>
+// a row, read(x, inside) (x is a cell of the row either way, so that every load
+// can be in flight at once), col(kx) the column store of kx.  buf is free on return.
+template <int FB, class PL, class SRC, class COL>
 __device__ __forceinline__ void rows_forward(PL pl, const ConvDev &c, double2 *buf, int p0, int np, SRC src, COL col)
 {
     const int hp = (c.Y + 1) >> 1;
-    fft_batch<true, false>(
+    fft_batch<true, false, 0>(
         pl, c.twx, buf, np,
         [&](int f) {
             const int p = p0 + f, z = p / hp, y = 2 * (p - z * hp), X = c.X;
             const bool two = y + 1 < c.Y;
             const auto ra = src(z, y), rb = src(z, two ? y + 1 : y);
             return [=](int x) {
-                double2 v = make_double2(0.0, 0.0);
-                if (x < X) {
-                    v.x = (double)ra(x);
-                    if (two) v.y = (double)rb(x);
-                }
-                return v;
+                const bool in = x < X;
+                const int xx = in ? x : X - 1;
+                const double a = (double)ra(xx, in), b = (double)rb(xx, in && two);
+                return make_double2(in ? a : 0.0, in && two ? b : 0.0);
             };
         },
         [](int) { return [](int, double2) {}; });
     __syncthreads();
-    for (int e = threadIdx.x; e < np * c.hx; e += blockDim.x) {
-        const int k = e / np, f = e - k * np;
+    for (int e = threadIdx.x; e < FB * (PL::n / 2 + 1); e += blockDim.x) {
+        const int k = e / FB, f = e % FB;
+        if (f >= np) continue;
         const int kn = k ? PL::n - k : 0;
         const double2 *t = buf + f * PL::stride;
         const double2 a = t[k + (k >> PL::shift)], b = t[kn + (kn >> PL::shift)];
@@ -317,6 +422,40 @@ __device__ __forceinline__ void rows_forward(PL pl, const ConvDev &c, double2 *b
     __syncthreads();
 }
 
+// The layers' spectra of nc columns times Ghat, real and imaginary parts
+// exchanged (the next transform goes back).  ZM: the layers, or their bound.
+template <class PL, int ZM, class KX>
+__device__ __forceinline__ void times_kernel(const ConvDev &c, double2 *buf, int nc, KX kx)
+{
+    const int Z = ZM == ZMAX ? c.Z : ZM;
+    for (int e = threadIdx.x; e < nc * PL::n; e += blockDim.x) {
+        const int j = e / PL::n, ky = e % PL::n, kk = min(ky, PL::n - ky);
+        const double *g = c.G + (long long)kx(j) * Z * c.hy + kk;
+        double2 *v = buf + j * Z * PL::stride + ky + (ky >> PL::shift);
+        double gv[ZM];
+        double2 a[ZM];
+#pragma unroll
+        for (int z = 0; z < ZM; z++)
+            if (z < Z) {
+                gv[z] = __ldg(g + z * c.hy);
+                a[z] = v[z * PL::stride];
+            }
+#pragma unroll
+        for (int z = 0; z < ZM; z++)
+            if (z < Z) {
+                double2 s = make_double2(0.0, 0.0);
+#pragma unroll
+                for (int w = 0; w < ZM; w++)
+                    if (w < Z) {
+                        const double gg = gv[z > w ? z - w : w - z];
+                        s.x = fma(gg, a[w].x, s.x);
+                        s.y = fma(gg, a[w].y, s.y);
+                    }
+                v[z * PL::stride] = make_double2(s.y, s.x);
+            }
+    }
+}
+
 // The Z columns of each of nc columns (col(j), kx(j)): forward, times Ghat,
 // back, in the column store.  nc Z padded transforms in buf; groups of whole
 // transforms that fit the CTA one butterfly per thread.
@@ -326,45 +465,29 @@ __device__ __forceinline__ void columns(PL pl, const ConvDev &c, double2 *buf, i
     const int Z = c.Z, Y = c.Y, ys = c.ys;
     const int nf = nc * Z, per = min(nf, max(1, (int)blockDim.x / PL::mmax));
     for (int f0 = 0; f0 < nf; f0 += per)
-        fft_batch<true, false>(
+        fft_batch<true, false, 0>(
             pl, c.twy, buf + f0 * PL::stride, min(per, nf - f0),
             [&](int f) {
                 const int j = (f0 + f) / Z, z = f0 + f - j * Z;
                 const double2 *p = col(j) + z * ys;
-                return [=](int y) { return y < Y ? p[y] : make_double2(0.0, 0.0); };
+                return [=](int y) {
+                    const double2 a = p[min(y, Y - 1)];
+                    return make_double2(y < Y ? a.x : 0.0, y < Y ? a.y : 0.0);
+                };
             },
             [](int) { return [](int, double2) {}; });
     __syncthreads();
-    for (int e = threadIdx.x; e < nc * PL::n; e += blockDim.x) {
-        const int j = e / PL::n, ky = e % PL::n, kk = min(ky, PL::n - ky);
-        const double *g = c.G + (long long)kx(j) * Z * c.hy + kk;
-        double2 *v = buf + j * Z * PL::stride + ky + (ky >> PL::shift);
-        double gv[ZMAX];
-        double2 a[ZMAX];
-#pragma unroll
-        for (int z = 0; z < ZMAX; z++)
-            if (z < Z) {
-                gv[z] = __ldg(g + z * c.hy);
-                a[z] = v[z * PL::stride];
-            }
-#pragma unroll
-        for (int z = 0; z < ZMAX; z++)
-            if (z < Z) {
-                double2 s = make_double2(0.0, 0.0);
-#pragma unroll
-                for (int w = 0; w < ZMAX; w++)
-                    if (w < Z) {
-                        const double gg = gv[z > w ? z - w : w - z];
-                        s.x = fma(gg, a[w].x, s.x);
-                        s.y = fma(gg, a[w].y, s.y);
-                    }
-                v[z * PL::stride] = make_double2(s.y, s.x);  // exchanged: the next transform goes back
-            }
+    switch (Z) {
+    case 1: times_kernel<PL, 1>(c, buf, nc, kx); break;
+    case 2: times_kernel<PL, 2>(c, buf, nc, kx); break;
+    case 3: times_kernel<PL, 3>(c, buf, nc, kx); break;
+    case 4: times_kernel<PL, 4>(c, buf, nc, kx); break;
+    default: times_kernel<PL, ZMAX>(c, buf, nc, kx); break;
     }
     __syncthreads();
     for (int f0 = 0; f0 < nf; f0 += per) {
         double2 *b0 = buf + f0 * PL::stride;
-        fft_batch<false, true>(
+        fft_batch<false, true, 0>(
             pl, c.twy, b0, min(per, nf - f0),
             [=](int f) {
                 const double2 *p = b0 + f * PL::stride;
@@ -382,11 +505,11 @@ __device__ __forceinline__ void columns(PL pl, const ConvDev &c, double2 *buf, i
 }
 
 // Rows back for pairs p0 .. p0 + np - 1: dst(z, y) gives a writer of phi's row.
-template <class PL, class COL, class DST>
+template <int FB, class PL, class COL, class DST>
 __device__ __forceinline__ void rows_back(PL pl, const ConvDev &c, double2 *buf, int p0, int np, COL col, DST dst)
 {
     const int hp = (c.Y + 1) >> 1;
-    fft_batch<false, false>(
+    fft_batch<false, false, FB>(
         pl, c.twx, buf, np,
         [&](int f) {
             const int p = p0 + f, z = p / hp, y = 2 * (p - z * hp), o = z * c.ys + y;

@@ -6,7 +6,11 @@
 // cells; an offset table gives each instance's first cell and dims, and a tile
 // table cuts every instance into <= 256-cell tiles that never cross an
 // instance, so the per-cell kernels (divergence, field + LLG + RK4 stage) are
-// one launch over all tiles.  The exact potential is one launch over
+// one launch over all tiles.  The exact potential is a convolution (conv.cuh)
+// in three launches over (instance, row pairs) and (instance, columns) items;
+// ensembles with an instance it does not serve (more than 8 layers, more than
+// 256 cells along y) or without memory for its column store take the pair sum,
+// one launch over
 // (instance, block of target rows) items: several short target rows share a
 // warp, each lane keeps 8 consecutive targets in registers and slides a window
 // over a mirrored table G[|dz|][|dy|][.] = dV/|r| kept in shared memory, with
@@ -19,8 +23,11 @@
 #include <string.h>
 
 #include <algorithm>
+#include <map>
+#include <tuple>
 #include <vector>
 
+#include "conv.cuh"
 #include "mms_internal.cuh"
 #include "stencil_dev.cuh"
 
@@ -110,30 +117,27 @@ __global__ void __launch_bounds__(ETPB) k_ens_div(const double *__restrict__ M, 
   }
 }
 
-// one RK4 stage for every instance (see k_rk4_stage in stencil.cu)
+// one RK4 stage for every instance (see k_rk4_stage in stencil.cu), over the
+// tiles that hold material: a film's empty layers cost nothing.  The last CTA
+// of stage 3 advances the time.
 __global__ void __launch_bounds__(ETPB) k_ens_stage(const float *__restrict__ phi, const double *__restrict__ Mst,
                                                     double *__restrict__ M, double *__restrict__ K,
                                                     double *__restrict__ Mnext, const uint8_t *__restrict__ mat,
-                                                    const double *__restrict__ tstate, const EnsInst *__restrict__ inst,
-                                                    const EnsTile *__restrict__ tiles, double *__restrict__ flag,
-                                                    int ntiles, long long Ntot, double dx, double dy, double dz,
-                                                    PhysK p, int stage)
+                                                    double *__restrict__ tstate, const EnsInst *__restrict__ inst,
+                                                    const EnsTile *__restrict__ tiles, const int *__restrict__ ntiles,
+                                                    double *__restrict__ flag, long long Ntot, double dx, double dy,
+                                                    double dz, PhysK p, int stage)
 {
-  for (int tix = blockIdx.x; tix < ntiles; tix += gridDim.x) {
+  pdl_begin();
+  const double dt = tstate[TIME_DT];
+  for (int tix = blockIdx.x; tix < *ntiles; tix += gridDim.x) {
     const EnsTile tl = tiles[tix];
     if ((int)threadIdx.x >= tl.count) continue;
     const EnsInst in = inst[tl.inst];
     const long long i = tl.start + threadIdx.x;   // within the instance
     const long long gi = in.off + i;              // global cell
     const long long N = Ntot;
-    if (!mat[gi]) {
-        double *dst = (stage < 3) ? Mnext : M;
-        dst[gi] = 0.0;
-        dst[gi + N] = 0.0;
-        dst[gi + 2 * N] = 0.0;
-        continue;
-    }
-    const double dt = tstate[TIME_DT];
+    if (!mat[gi]) continue;  // M and the stage buffers are zero there
     const GridK g = inst_grid(in, Ntot, dx, dy, dz);
     int x, y, z;
     const long long plane = (long long)in.X * in.Y;
@@ -142,7 +146,7 @@ __global__ void __launch_bounds__(ETPB) k_ens_stage(const float *__restrict__ ph
     z = (int)(i / plane);
     const double he[3] = {p.external ? in.hx : 0.0, p.external ? in.hy : 0.0, p.external ? in.hz : 0.0};
     double h[3];
-    field_soa(phi + in.off, Mst + in.off, i, x, y, z, g, p, he, h);
+    field_soa<true>(phi + in.off, Mst + in.off, i, x, y, z, g, p, he, h);
     const double ms[3] = {Mst[gi], Mst[gi + N], Mst[gi + 2 * N]};
     double k[3];
     llg(ms, h, p, k);
@@ -175,13 +179,110 @@ __global__ void __launch_bounds__(ETPB) k_ens_stage(const float *__restrict__ ph
         M[gi + N] = n1;
         M[gi + 2 * N] = n2;
     }
+  }  if (stage != 3) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+      unsigned *ctr = reinterpret_cast<unsigned *>(tstate + TIME_CTR);
+      if (atomicAdd(ctr, 1u) == gridDim.x - 1) {
+          tstate[TIME_TK1] = tstate[TIME_T];
+          tstate[TIME_T] += dt;
+          *ctr = 0u;
+      }
   }
 }
 
-__global__ void k_ens_advance(double *tstate)
+// ---- the exact potential of every instance as a convolution (conv.cuh) ---------
+// The three passes over all instances, CTA = some row pairs or columns of one
+// instance; the items are ordered by transform length, so that neighbouring
+// CTAs run the same code.  512 instances of 16 .. 64 x 16 .. 64 x 3 (2.34 M
+// cells): 120 us a potential (rows 46, columns 69, back 22 us cold) against
+// 770 us for the pair sum, 602 us a step against 3,973.  Bound by the latency of
+// the passes: 14 to 20 warps an SM at 92 to 128 registers, issue 23 to 31 %,
+// FP64 pipe 9 to 22 %, L2 20 %.  A cluster of CTAs per instance with the
+// columns in distributed shared memory (a whole step in one launch) took 767
+// us a step: its few warps work through long instruction streams alone.
+constexpr int CONV_THREADS = 64;  // 128: 936 us a step of 512 instances against 782
+constexpr int CONV_PAIRS = 8;     // row pairs per CTA at most (4: 729 against 710)
+
+struct EnsConv {
+    mmsconv::ConvDev c;
+    long long off;    // first cell in the planes
+    long long store;  // first element in the column store
+};
+
+struct ConvItem {
+    int inst, first;  // first row pair or column
+};
+
+__global__ void __launch_bounds__(CONV_THREADS) k_ens_rows(const double *__restrict__ M,
+                                                           const EnsConv *__restrict__ conv,
+                                                           const ConvItem *__restrict__ items, long long Ntot,
+                                                           DivScale h, double2 *__restrict__ store)
 {
-    tstate[TIME_TK1] = tstate[TIME_T];
-    tstate[TIME_T] += tstate[TIME_DT];
+    extern __shared__ __align__(16) double2 cbuf[];
+    __shared__ EnsConv in;
+    const ConvItem it = items[blockIdx.x];
+    for (int i = threadIdx.x; i < (int)(sizeof(EnsConv) / 4); i += CONV_THREADS)
+        reinterpret_cast<int *>(&in)[i] = __ldg(reinterpret_cast<const int *>(conv + it.inst) + i);
+    __syncthreads();
+    pdl_begin();  // the tables are constant; the state is the predecessor's output
+    const mmsconv::ConvDev &c = in.c;
+    const GridK g = {c.X, c.Y, c.Z, Ntot, 0, 0, 0};
+    const double *m = M + in.off;
+    double2 *st = store + in.store;
+    const int cs = c.cs, np = c.Z * ((c.Y + 1) >> 1) - it.first;
+    mmsconv::with_batch_plan(c.px.id, [&](auto pl) {
+        mmsconv::rows_forward<mmsconv::row_pairs<decltype(pl)>(CONV_THREADS, CONV_PAIRS)>(
+            pl, c, cbuf, it.first, min(c.fb, np),
+            [=](int z, int y) {
+                return [=](int x, bool) { return div_soa_cell<true>(m, (z * g.Y + y) * g.X + x, x, y, z, g, h); };
+            },
+            [=](int k) { return st + k * cs; });
+    });
+}
+
+__global__ void __launch_bounds__(CONV_THREADS, 8) k_ens_columns(const EnsConv *__restrict__ conv,
+                                                              const ConvItem *__restrict__ items,
+                                                              double2 *__restrict__ store)
+{
+    extern __shared__ __align__(16) double2 cbuf[];
+    __shared__ EnsConv in;
+    const ConvItem it = items[blockIdx.x];
+    for (int i = threadIdx.x; i < (int)(sizeof(EnsConv) / 4); i += CONV_THREADS)
+        reinterpret_cast<int *>(&in)[i] = __ldg(reinterpret_cast<const int *>(conv + it.inst) + i);
+    __syncthreads();
+    pdl_begin();
+    const mmsconv::ConvDev &c = in.c;
+    double2 *st = store + in.store + (long long)it.first * c.cs;
+    const int cs = c.cs, k0 = it.first;
+    mmsconv::with_batch_plan(c.py.id, [&](auto pl) {
+        mmsconv::columns(pl, c, cbuf, min(c.cpg, c.hx - k0), [=](int j) { return st + j * cs; },
+                                        [=](int j) { return k0 + j; });
+    });
+}
+
+__global__ void __launch_bounds__(CONV_THREADS) k_ens_back(const EnsConv *__restrict__ conv,
+                                                           const ConvItem *__restrict__ items,
+                                                           const double2 *__restrict__ store, float *__restrict__ phi)
+{
+    extern __shared__ __align__(16) double2 cbuf[];
+    __shared__ EnsConv in;
+    const ConvItem it = items[blockIdx.x];
+    for (int i = threadIdx.x; i < (int)(sizeof(EnsConv) / 4); i += CONV_THREADS)
+        reinterpret_cast<int *>(&in)[i] = __ldg(reinterpret_cast<const int *>(conv + it.inst) + i);
+    __syncthreads();
+    pdl_begin();
+    const mmsconv::ConvDev &c = in.c;
+    const double2 *st = store + in.store;
+    float *ph = phi + in.off;
+    const int cs = c.cs, X = c.X, Y = c.Y, np = c.Z * ((c.Y + 1) >> 1) - it.first;
+    mmsconv::with_batch_plan(c.px.id, [&](auto pl) {
+        mmsconv::rows_back<mmsconv::row_pairs<decltype(pl)>(CONV_THREADS, CONV_PAIRS)>(pl, c, cbuf, it.first, min(c.fb, np), [=](int k) { return st + k * cs; },
+                           [=](int z, int y) {
+                               float *r = ph + (z * Y + y) * X;
+                               return [=](int x, float v) { r[x] = v; };
+                           });
+    });
 }
 
 __global__ void k_ens_set_dt(double *tstate, double dt) { tstate[TIME_DT] = dt; }
@@ -340,6 +441,15 @@ struct mms_ens {
     int grid_direct = 0, grid_cells = 0;
     unsigned *next = nullptr;         // work counter of the persistent direct kernel
     std::vector<EnsInst> hin;         // host copy of the offset table
+    std::vector<EnsTile> htiles;      // and of the tile table
+    EnsTile *mtiles = nullptr;        // the tiles that hold material, and their number
+    int *nmtiles = nullptr;
+    // the exact potential as a convolution; conv == NULL: the pair sum
+    EnsConv *conv = nullptr;
+    ConvItem *row_items = nullptr, *col_items = nullptr;
+    double2 *store = nullptr;
+    int nrow_items = 0, ncol_items = 0;
+    size_t conv_smem = 0;
     int64_t launches = 0;
     size_t dev_bytes = 0;
     EnsInst *inst = nullptr;
@@ -456,13 +566,11 @@ int ens_set_shape(mms_ens *e, int ew, int qrows)
             MMS_CUDA_TRY(cudaFuncSetAttribute(k_ens_direct, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               (int)e->direct_smem));
     }
-    int dev = 0, sms = 0, per = 0, perc = 0;
+    int dev = 0, sms = 0, per = 0;
     MMS_CUDA_TRY(cudaGetDevice(&dev));
     MMS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     MMS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_ens_direct, ew * 32, e->direct_smem));
-    MMS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perc, k_ens_stage, ETPB, 0));
     e->grid_direct = std::max(1, std::min(e->nitems, std::max(per, 1) * sms));
-    e->grid_cells = std::max(1, std::min(e->ntiles, std::max(perc, 1) * sms));
     if (e->exec) {  // a captured step holds the old launch shape
         cudaGraphExecDestroy(e->exec);
         e->exec = nullptr;
@@ -484,9 +592,26 @@ int ens_direct(mms_ens *e)
     return MMS_OK;
 }
 
+int ens_conv(mms_ens *e, const double *Mst)
+{
+    MMS_CUDA_TRY(launch_k(k_ens_rows, dim3(e->nrow_items), dim3(CONV_THREADS), e->conv_smem, e->stream, Mst,
+                          (const EnsConv *)e->conv, (const ConvItem *)e->row_items, e->Ntot,
+                          div_scale(e->dx, e->dy, e->dz), e->store));
+    ENS_LAUNCH_CHECK(e);
+    MMS_CUDA_TRY(launch_k(k_ens_columns, dim3(e->ncol_items), dim3(CONV_THREADS), e->conv_smem, e->stream,
+                          (const EnsConv *)e->conv, (const ConvItem *)e->col_items, e->store));
+    ENS_LAUNCH_CHECK(e);
+    MMS_CUDA_TRY(launch_k(k_ens_back, dim3(e->nrow_items), dim3(CONV_THREADS), e->conv_smem, e->stream,
+                          (const EnsConv *)e->conv, (const ConvItem *)e->row_items, (const double2 *)e->store,
+                          e->phi));
+    ENS_LAUNCH_CHECK(e);
+    return MMS_OK;
+}
+
 int ens_potential(mms_ens *e, const double *Mst)
 {
     if (!e->p.demag) return MMS_OK;
+    if (e->conv) return ens_conv(e, Mst);
     k_ens_div<<<e->grid_cells, ETPB, 0, e->stream>>>(Mst, e->rho, e->inst, e->tiles, e->ntiles, e->Ntot, e->dx, e->dy,
                                                      e->dz, div_scale(e->dx, e->dy, e->dz));
     ENS_LAUNCH_CHECK(e);
@@ -495,9 +620,10 @@ int ens_potential(mms_ens *e, const double *Mst)
 
 int ens_stage(mms_ens *e, int stage, const double *Mst, double *Mnext)
 {
-    k_ens_stage<<<e->grid_cells, ETPB, 0, e->stream>>>(e->phi, Mst, e->M, e->K, Mnext, e->mat, e->tstate, e->inst,
-                                                       e->tiles, e->flag, e->ntiles, e->Ntot, e->dx, e->dy, e->dz,
-                                                       e->pk(), stage);
+    MMS_CUDA_TRY(launch_k(k_ens_stage, dim3(e->grid_cells), dim3(ETPB), 0, e->stream, (const float *)e->phi, Mst, e->M,
+                          e->K, Mnext, (const uint8_t *)e->mat, e->tstate, (const EnsInst *)e->inst,
+                          (const EnsTile *)e->mtiles, (const int *)e->nmtiles, e->flag, e->Ntot, e->dx, e->dy, e->dz,
+                          e->pk(), stage));
     ENS_LAUNCH_CHECK(e);
     return MMS_OK;
 }
@@ -512,8 +638,91 @@ int ens_step(mms_ens *e)
     MMS_TRY(ens_potential(e, e->A));
     MMS_TRY(ens_stage(e, 3, e->A, nullptr));
     MMS_TRY(ens_potential(e, e->M));
-    k_ens_advance<<<1, 1, 0, e->stream>>>(e->tstate);
-    ENS_LAUNCH_CHECK(e);
+    return MMS_OK;
+}
+
+// The convolution's tables (one per pair of transform lengths and layers), the
+// items and the column store.  Leaves e->conv NULL, for the pair sum, where an
+// instance has no plan or there is no memory.
+int ens_conv_prepare(mms_ens *e)
+{
+    using namespace mmsconv;
+    std::vector<EnsConv> conv(e->n);
+    std::map<std::tuple<int, int, int>, size_t> tables;  // offset of each in the allocation
+    size_t bytes = 0, scratch = 0, smem = 0;
+    long long store = 0;
+    std::vector<std::pair<int, ConvItem>> rows, cols;  // with the transform length
+    for (int i = 0; i < e->n; i++) {
+        ConvDev &c = conv[i].c;
+        size_t s = 0;
+        if (!conv_layout(c, e->hin[i].X, e->hin[i].Y, e->hin[i].Z, NBATCH, CONV_THREADS, CONV_PAIRS, &s))
+            return MMS_OK;
+        smem = std::max(smem, s);
+        conv[i].off = e->hin[i].off;
+        conv[i].store = store;
+        store += (long long)c.hx * c.cs;
+        const int pairs = c.Z * ((c.Y + 1) / 2);
+        for (int p = 0; p < pairs; p += c.fb) rows.push_back({c.px.n, {i, p}});
+        for (int k = 0; k < c.hx; k += c.cpg) cols.push_back({c.py.n, {i, k}});
+        if (tables.try_emplace({c.px.id, c.py.id, c.Z}, bytes).second) {
+            bytes += conv_table_bytes(c);
+            scratch = std::max(scratch, conv_table_scratch(c));
+        }
+    }
+    std::vector<ConvItem> items;
+    for (auto *v : {&rows, &cols}) {
+        std::stable_sort(v->begin(), v->end(), [](const auto &a, const auto &b) { return a.first > b.first; });
+        for (auto &p : *v) items.push_back(p.second);
+    }
+    // one allocation: instances, items, tables, column store (first the tables' scratch)
+    const size_t at_items = (conv.size() * sizeof(EnsConv) + 255) / 256 * 256;
+    const size_t at_tables = at_items + (items.size() * sizeof(ConvItem) + 255) / 256 * 256;
+    const size_t at_store = at_tables + bytes;
+    const size_t total = at_store + std::max(scratch, (size_t)store * sizeof(double2));
+    char *mem = nullptr;
+    if (cudaMalloc((void **)&mem, total) != cudaSuccess) {
+        cudaGetLastError();  // not an error of the call: the pair sum needs no store
+        return MMS_OK;
+    }
+    e->conv = (EnsConv *)mem;  // (freed with the ensemble)
+    e->dev_bytes += total;
+    e->row_items = (ConvItem *)(mem + at_items);
+    e->col_items = e->row_items + rows.size();
+    e->nrow_items = (int)rows.size();
+    e->ncol_items = (int)cols.size();
+    e->store = (double2 *)(mem + at_store);
+    e->conv_smem = smem;
+    std::map<size_t, ConvDev> built;
+    for (EnsConv &v : conv) {
+        const size_t at = tables.at({v.c.px.id, v.c.py.id, v.c.Z});
+        auto b = built.find(at);
+        if (b == built.end()) {
+            MMS_TRY(conv_build_tables(v.c, mem + at_tables + at, (double *)(mem + at_store), e->dx, e->dy, e->dz,
+                                      e->stream, &e->launches));
+            b = built.emplace(at, v.c).first;
+        }
+        v.c.twx = b->second.twx;
+        v.c.twy = b->second.twy;
+        v.c.G = b->second.G;
+    }
+    MMS_CUDA_TRY(cudaMemcpyAsync(e->conv, conv.data(), conv.size() * sizeof(EnsConv), cudaMemcpyHostToDevice, e->stream));
+    MMS_CUDA_TRY(cudaMemcpyAsync(e->row_items, items.data(), items.size() * sizeof(ConvItem), cudaMemcpyHostToDevice,
+                                 e->stream));
+    MMS_CUDA_TRY(cudaStreamSynchronize(e->stream));
+    MMS_TRY(conv_raise_smem((const void *)k_ens_rows, smem));
+    MMS_TRY(conv_raise_smem((const void *)k_ens_columns, smem));
+    MMS_TRY(conv_raise_smem((const void *)k_ens_back, smem));
+    return MMS_OK;
+}
+
+// the persistent grid of the cell kernels
+int ens_cell_grid(mms_ens *e)
+{
+    int dev = 0, sms = 0, per = 0;
+    MMS_CUDA_TRY(cudaGetDevice(&dev));
+    MMS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    MMS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_ens_stage, ETPB, 0));
+    e->grid_cells = std::max(1, std::min(e->ntiles, std::max(per, 1) * sms));
     return MMS_OK;
 }
 
@@ -591,6 +800,7 @@ int mms_ens_create(const mms_ens_instance *inst, int n, double dx, double dy, do
         e->ntiles = (int)htiles.size();
         e->nitems = 0;
         e->hin = hin;
+        e->htiles = htiles;
         if (stream) {
             e->stream = (cudaStream_t)stream;
         } else {
@@ -604,9 +814,9 @@ int mms_ens_create(const mms_ens_instance *inst, int n, double dx, double dy, do
         const size_t N = (size_t)Ntot;
         if ((st = ens_alloc(e, &e->inst, (size_t)n))) break;
         if ((st = ens_alloc(e, &e->tiles, htiles.size()))) break;
+        if ((st = ens_alloc(e, &e->mtiles, htiles.size()))) break;
+        if ((st = ens_alloc(e, &e->nmtiles, 1))) break;
         if ((st = ens_alloc(e, &e->next, 1))) break;
-        if ((st = ens_alloc(e, &e->gtab, (size_t)ts.Z * ts.Ym * ts.pitch))) break;
-        if ((st = ens_alloc(e, &e->rho, N))) break;
         if ((st = ens_alloc(e, &e->phi, N))) break;
         if ((st = ens_alloc(e, &e->mat, N))) break;
         if ((st = ens_alloc(e, &e->M, 3 * N))) break;
@@ -629,9 +839,15 @@ int mms_ens_create(const mms_ens_instance *inst, int n, double dx, double dy, do
             st = MMS_ERR_CUDA;
             break;
         }
-        const long long tn = (long long)ts.Z * ts.Ym * ts.pitch;
-        k_ens_table<<<div_up(tn, 256), 256, 0, e->stream>>>(e->gtab, ts, dx, dy, dz);
-        if ((st = ens_set_shape(e, 8, 16))) break;
+        if ((st = ens_cell_grid(e))) break;
+        if ((st = ens_conv_prepare(e))) break;
+        if (!e->conv) {
+            const long long tn = (long long)ts.Z * ts.Ym * ts.pitch;
+            if ((st = ens_alloc(e, &e->gtab, (size_t)tn))) break;
+            if ((st = ens_alloc(e, &e->rho, N))) break;
+            k_ens_table<<<div_up(tn, 256), 256, 0, e->stream>>>(e->gtab, ts, dx, dy, dz);
+            if ((st = ens_set_shape(e, 8, 16))) break;
+        }
         if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(e->stream) != cudaSuccess) {
             mms_set_error("ensemble set-up failed: %s", cudaGetErrorString(cudaGetLastError()));
             st = MMS_ERR_CUDA;
@@ -657,7 +873,7 @@ int mms_ens_destroy(mms_ens *e)
     if (e->exec) cudaGraphExecDestroy(e->exec);
     if (e->graph) cudaGraphDestroy(e->graph);
     void *b[] = {e->inst, e->tiles, e->items, e->gtab, e->rho, e->phi, e->mat, e->M, e->A, e->B, e->K, e->tstate,
-                 e->flag, e->next};
+                 e->flag, e->next, e->mtiles, e->nmtiles, e->conv};
     for (void *p : b)
         if (p) cudaFree(p);
     if (e->h_scratch) cudaFreeHost(e->h_scratch);
@@ -681,6 +897,17 @@ int mms_ens_state_set(mms_ens *e, const uint8_t *material, const double *M)
     MMS_CUDA_TRY(cudaMemcpyAsync(e->K, M, 3 * N * sizeof(double), cudaMemcpyHostToDevice, e->stream));
     k_aos_to_soa_ens<<<div_up(e->Ntot, 256), 256, 0, e->stream>>>(e->K, e->mat, e->M, e->Ntot);
     ENS_LAUNCH_CHECK(e);
+    // the stage kernels visit the material cells alone: the others stay zero
+    MMS_CUDA_TRY(cudaMemsetAsync(e->A, 0, 3 * N * sizeof(double), e->stream));
+    MMS_CUDA_TRY(cudaMemsetAsync(e->B, 0, 3 * N * sizeof(double), e->stream));
+    std::vector<EnsTile> mt;
+    for (const EnsTile &t : e->htiles) {
+        const uint8_t *m = material + e->hin[t.inst].off + t.start;
+        if (std::any_of(m, m + t.count, [](uint8_t v) { return v != 0; })) mt.push_back(t);
+    }
+    const int nmt = (int)mt.size();
+    MMS_CUDA_TRY(cudaMemcpyAsync(e->mtiles, mt.data(), mt.size() * sizeof(EnsTile), cudaMemcpyHostToDevice, e->stream));
+    MMS_CUDA_TRY(cudaMemcpyAsync(e->nmtiles, &nmt, sizeof(int), cudaMemcpyHostToDevice, e->stream));
     MMS_CUDA_TRY(cudaMemsetAsync(e->tstate, 0, TIME_SLOTS * sizeof(double), e->stream));
     MMS_CUDA_TRY(cudaMemsetAsync(e->flag, 0, sizeof(double), e->stream));
     MMS_CUDA_TRY(cudaStreamSynchronize(e->stream));
@@ -766,13 +993,33 @@ int mms_ens_autotune(mms_ens *e, int reps, int *ew, int *qrows, double *best_ms)
         mms_set_error("mms_ens_autotune: ensemble state not set or reps < 1");
         return MMS_ERR_NOT_READY;
     }
+    cudaEvent_t e0, e1;
+    MMS_CUDA_TRY(cudaEventCreate(&e0));
+    MMS_CUDA_TRY(cudaEventCreate(&e1));
+    if (e->conv) {  // no shape to choose: the time of one potential
+        int st = ens_conv(e, e->M);  // warm
+        cudaEventRecord(e0, e->stream);
+        for (int r = 0; r < reps && st == MMS_OK; r++) st = ens_conv(e, e->M);
+        cudaEventRecord(e1, e->stream);
+        float ms = 0.f;
+        if (st == MMS_OK && cudaEventSynchronize(e1) != cudaSuccess) {
+            mms_set_error("mms_ens_autotune: %s", cudaGetErrorString(cudaGetLastError()));
+            st = MMS_ERR_CUDA;
+        }
+        if (st == MMS_OK) cudaEventElapsedTime(&ms, e0, e1);
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        MMS_TRY(st);
+        e->phi_valid = false;
+        if (ew) *ew = e->ew;
+        if (qrows) *qrows = e->qrows;
+        if (best_ms) *best_ms = ms / reps;
+        return MMS_OK;
+    }
     // the charges of the current state
     k_ens_div<<<e->grid_cells, ETPB, 0, e->stream>>>(e->M, e->rho, e->inst, e->tiles, e->ntiles, e->Ntot, e->dx, e->dy,
                                                      e->dz, div_scale(e->dx, e->dy, e->dz));
     ENS_LAUNCH_CHECK(e);
-    cudaEvent_t e0, e1;
-    MMS_CUDA_TRY(cudaEventCreate(&e0));
-    MMS_CUDA_TRY(cudaEventCreate(&e1));
     const int ews[] = {4, 8, 16}, qs[] = {8, 16, 32};
     double best = 1e30;
     int bew = e->ew, bq = e->qrows, st = MMS_OK;

@@ -166,3 +166,52 @@ def test_c4_512_instances_5000_steps(cuda, lib):
         worst = max(worst, a)
         assert a < 1e-3, (i, dims[i], a)
     print(f"C4 5000 steps: max angle vs single contexts {worst:.2e} deg")
+
+
+@pytest.mark.parametrize("kind", ["along x", "along y", "layers", "pair sum"])
+def test_ensemble_at_the_edges_of_its_plans(cuda, lib, oracle_mod, kind):
+    """Instances at both sides of every transform length of the batched
+    convolution (2 n - 1 <= length), odd and lone rows, 1 .. 8 layers; and an
+    ensemble with a 9-layer instance, which takes the pair sum.  Two steps
+    against the FP64 oracle: phi rounded to FP32 turns M by about
+    gamma dt H 2^-24 = 1e-9 rad an evaluation; bound 1e-5 deg (1.7e-7 rad),
+    which leaves room for arccos near 1."""
+    import mmsb200
+    from mmsb200 import geometry
+    from mmsb200.ensemble import Ensemble
+    sides = (1, 2, 8, 9, 16, 17, 24, 25, 32, 33, 40, 41, 48, 49, 64, 65, 80, 81, 96, 97, 128, 129, 160, 161, 256)
+    dims = {"along x": [(n, 5, 3) for n in sides], "along y": [(6, n, 3) for n in sides[:-3]],
+            "layers": [(11, 7, z) for z in range(1, 9)], "pair sum": [(11, 7, 3), (12, 5, 9)]}[kind]
+    masks = [geometry.rectangle(*t, layers="all") for t in dims]
+    Ms = [geometry.random_sphere(m, 40 + i) for i, m in enumerate(masks)]
+    with Ensemble(dims, D, mmsb200.make_params()) as ens:
+        ens.state_set(masks, Ms)
+        ens.run_fixed(1e-13, 2)
+        out, _ = ens.state_get()
+    for i, (X, Y, Z) in enumerate(dims):
+        ref = oracle_mod.rk4_run(oracle_mod.Grid(X, Y, Z, *D), oracle_mod.Params(), masks[i], Ms[i], 1e-13, 2)
+        assert max_angle_deg(out[i], ref, masks[i]) < 1e-5, dims[i]
+
+
+def test_ensemble_state_set_again_with_another_mask(cuda, lib):
+    """the stage kernels visit material tiles alone: a second state with other
+    material must not see the first one's"""
+    import mmsb200
+    from mmsb200 import geometry
+    from mmsb200.ensemble import Ensemble
+    dims = [(24, 16, 3), (17, 19, 3)]
+    a = [geometry.rectangle(*t) for t in dims]
+    b = [geometry.disc(*t, 5) for t in dims]
+    Ma = [geometry.random_sphere(m, 1 + i) for i, m in enumerate(a)]
+    Mb = [geometry.random_sphere(m, 7 + i) for i, m in enumerate(b)]
+    with Ensemble(dims, D, mmsb200.make_params()) as ens:
+        ens.state_set(b, Mb)
+        ens.run_fixed(1e-13, 3)
+        fresh, _ = ens.state_get()
+        ens.state_set(a, Ma)
+        ens.run_fixed(1e-13, 3)
+        ens.state_set(b, Mb)
+        ens.run_fixed(1e-13, 3)
+        again, _ = ens.state_get()
+    for x, y in zip(fresh, again):
+        assert np.array_equal(x, y)
