@@ -43,6 +43,7 @@ __global__ void k_splitk_reduce(const float *__restrict__ Cp, int splits, long l
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= MN) return;
     float v = Cp[i];
+#pragma unroll 8
     for (int s = 1; s < splits; s++) v += Cp[(long long)s * MN + i];
     C[i] = v;
 }
@@ -126,9 +127,15 @@ int umma_gemm_bf16_splitk(const void *A, int lda, const void *B, int ldb, float 
         return MMS_ERR_ARG;
     }
     const long long MN = (long long)M * N;
-    k_splitk_reduce<<<div_up(MN, 256), 256, 0, st>>>(Cpart, splits, MN, C);
+    k_splitk_reduce<<<div_up(MN, 64), 64, 0, st>>>(Cpart, splits, MN, C);
     MMS_CUDA_TRY(cudaGetLastError());
     return MMS_OK;
+}
+
+const int *umma_error_word()
+{
+    void *p = nullptr;
+    return cudaGetSymbolAddress(&p, g_umma_err) == cudaSuccess ? (const int *)p : nullptr;
 }
 
 int umma_check_error()

@@ -214,7 +214,8 @@ int umma_gemm_bf16(const void *A, int lda, const void *B, int ldb, float *C, int
 int umma_gemm_bf16_splitk_plan(int M, int N, int K, int bn, int *splits, int *kchunk);
 int umma_gemm_bf16_splitk(const void *A, int lda, const void *B, int ldb, float *C, float *Cpart, int M, int N,
                           int K, int bn, int splits, int kchunk, cudaStream_t st);
-int umma_check_error();
+int umma_check_error();            // reads and clears the core's error word
+const int *umma_error_word();      // its address on the current device
 
 // potential with the context's solver
 int launch_potential(mms_ctx *ctx, const float *rho, float *phi);

@@ -414,3 +414,30 @@ def test_time_potential_cli(cuda, lib):
     d = json.loads(r.stdout.strip().splitlines()[-1])
     assert d["network"]["rel_l2_vs_direct"] < 1e-4 < d["fmm"]["rel_l2_vs_direct"] < 1e-3
     assert d["network"]["us"] > 0 and d["fmm"]["us"] > 0
+
+
+@pytest.mark.parametrize("dims,batch", [((17, 17), 1), ((33, 20), 3), ((65, 130), 2), ((260, 20), 1)])
+def test_gradient_at_the_edges_of_its_levels(cuda, lib, oracle_mod, dims, batch):
+    """2, 3, 5 and 6 quadtree levels, ragged grids, odd batches (groups, chunks
+    and lines that end early): the gradient of a perturbed network against the
+    FP64 restatement, at the tolerances of test_gradient_matches_oracle"""
+    import torch
+    import mmsb200
+    from oracle import farnet as OF
+    w0 = _weights().astype(np.float64)
+    w = (w0 * (1 + 0.05 * np.random.default_rng(7).standard_normal(w0.size))).astype(np.float32)
+    X, Y = dims
+    u = _charges(X, tuple(range(3, 3 + batch)), oracle_mod, Y, "film").astype(np.float32)
+    far = np.stack([OF.forward(w0, b.astype(np.float64))[0] for b in u]).astype(np.float32)
+    nrm = np.array([(f.astype(np.float64) ** 2).sum() for f in far], np.float32)
+    lref, gref = OF.loss_and_gradient(w.astype(np.float64), [(u[b], far[b].astype(np.float64), float(nrm[b]))
+                                                             for b in range(batch)])
+    with mmsb200.FarNet(X, Y, batch=batch) as net:
+        net.set_weights(w)
+        loss, g = net.gradient(torch.from_numpy(u).cuda(), torch.from_numpy(far).cuda(), torch.from_numpy(nrm).cuda(),
+                               batch)
+        again = net.gradient(torch.from_numpy(u).cuda(), torch.from_numpy(far).cuda(), torch.from_numpy(nrm).cuda(),
+                             batch)[1]
+    assert abs(loss - lref) <= 1e-5 * lref, (loss, lref)
+    assert rel_l2(g, gref) < 1e-4
+    assert np.array_equal(g, again)
