@@ -172,6 +172,7 @@ int eval_state_potential(mms_ctx *ctx, const double *Mst)
     if (!ctx->p.demag) return MMS_OK;  // phi unused
     if (ctx->s.kind == MMS_SOLVER_FMM || (ctx->s.kind == MMS_SOLVER_SURROGATE && !ctx->sur_active))
         return launch_potential_fmm_state(ctx, Mst, ctx->rho, ctx->phi);
+    if (ctx->s.kind == MMS_SOLVER_DIRECT) return launch_potential_direct_state(ctx, Mst, ctx->phi);
     MMS_TRY(launch_divergence_soa(ctx, Mst, ctx->rho));
     MMS_TRY(launch_potential(ctx, ctx->rho, ctx->phi));
     return MMS_OK;
@@ -380,6 +381,20 @@ int mms_ctx_create(const mms_grid *grid, const mms_params *params, const mms_sol
             ctx->own_stream = true;
         }
         const size_t N = (size_t)ctx->N;
+        ctx->stat_blocks = (int)div_up(ctx->N, 256);
+        {
+            // the allocations below, each padded to 256 bytes; without memory
+            // for them in one piece they are tried one by one
+            const size_t sizes[] = {4 * N, 4 * N, 4 * N, 12 * N, 12 * N, N, 24 * N, 24 * N, 24 * N, 24 * N, 24 * N,
+                                    24 * N, TIME_SLOTS * 8, 4 * MMS_MAX_HEXT * 8, (size_t)ctx->stat_blocks * 64,
+                                    STAT_SLOTS * 8};
+            for (size_t b : sizes) ctx->arena_bytes += (b + 255) / 256 * 256;
+            if (!solver || solver->kind == MMS_SOLVER_DIRECT) ctx->arena_bytes += direct_bytes(*grid);
+            if (cudaMalloc((void **)&ctx->arena, ctx->arena_bytes) != cudaSuccess) {
+                cudaGetLastError();
+                ctx->arena = nullptr;
+            }
+        }
         if ((st = ctx_alloc(ctx, &ctx->rho, N))) break;
         if ((st = ctx_alloc(ctx, &ctx->phi, N))) break;
         if ((st = ctx_alloc(ctx, &ctx->phibak, N))) break;
@@ -394,7 +409,6 @@ int mms_ctx_create(const mms_grid *grid, const mms_params *params, const mms_sol
         if ((st = ctx_alloc(ctx, &ctx->Mfull, 3 * N))) break;
         if ((st = ctx_alloc(ctx, &ctx->tstate, TIME_SLOTS))) break;
         if ((st = ctx_alloc(ctx, &ctx->hext, 4 * MMS_MAX_HEXT))) break;
-        ctx->stat_blocks = (int)div_up(ctx->N, 256);
         if ((st = ctx_alloc(ctx, &ctx->stat_part, (size_t)ctx->stat_blocks * 8))) break;
         if ((st = ctx_alloc(ctx, &ctx->stats, STAT_SLOTS))) break;
         if (cudaMallocHost((void **)&ctx->h_stats, (STAT_SLOTS + TIME_SLOTS) * sizeof(double)) != cudaSuccess) {
@@ -447,11 +461,11 @@ int mms_ctx_destroy(mms_ctx *ctx)
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     drop_graph(ctx);
     fmm_plan_destroy(ctx);
-    conv_plan_destroy(ctx->conv);
-    void *bufs[] = {ctx->rho, ctx->phi, ctx->phibak, ctx->vecA, ctx->vecB, ctx->gtab, ctx->mat, ctx->M, ctx->A,
+    conv_plan_destroy(ctx);
+    void *bufs[] = {ctx->rho, ctx->phi, ctx->phibak, ctx->vecA, ctx->vecB, ctx->gtab, ctx->gsmall, ctx->mat, ctx->M, ctx->A,
                     ctx->B, ctx->K, ctx->Mbak, ctx->Mfull, ctx->tstate, ctx->hext, ctx->stat_part, ctx->stats};
-    for (void *b : bufs)
-        if (b) cudaFree(b);
+    for (void *b : bufs) ctx_free(ctx, b);
+    if (ctx->arena) cudaFree(ctx->arena);
     if (ctx->h_stats) cudaFreeHost(ctx->h_stats);
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
@@ -560,7 +574,9 @@ int mms_hfield_dev(mms_ctx *ctx, const float *M, float *H, float *charge, float 
     }
     float *rho = charge ? charge : ctx->rho;
     float *phi = potential ? potential : ctx->phi;
-    if (ctx->p.demag) {
+    if (ctx->p.demag && ctx->s.kind == MMS_SOLVER_DIRECT) {
+        MMS_TRY(launch_potential_direct_aos(ctx, M, charge, phi));
+    } else if (ctx->p.demag) {
         MMS_TRY(launch_divergence_aos(ctx, M, rho));
         MMS_TRY(launch_potential(ctx, rho, phi));
     }
@@ -591,7 +607,9 @@ int mms_hfield_host(mms_ctx *ctx, const float *M, float *H, float *charge, float
     }
     const size_t n = (size_t)ctx->N;
     MMS_CUDA_TRY(cudaMemcpyAsync(ctx->vecA, M, 3 * n * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
-    if (ctx->p.demag) {
+    if (ctx->p.demag && ctx->s.kind == MMS_SOLVER_DIRECT) {
+        MMS_TRY(launch_potential_direct_aos(ctx, ctx->vecA, charge ? ctx->rho : nullptr, ctx->phi));
+    } else if (ctx->p.demag) {
         MMS_TRY(launch_divergence_aos(ctx, ctx->vecA, ctx->rho));
         MMS_TRY(launch_potential(ctx, ctx->rho, ctx->phi));
     }

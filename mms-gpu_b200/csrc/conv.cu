@@ -74,30 +74,28 @@ __global__ void k_conv_table_y(const double *__restrict__ T, double *__restrict_
 // Three launches a potential.  Up to about 200 cells a side they are bound by
 // launch and barrier latency (4 us each), beyond by the column store's traffic
 // through L2 (32 bytes a cell and pass) and the FP64 passes.  Measured, whole
-// potential, against the pair sum: 64 x 64 x 3 13 us (100 us), 256 x 256 x 3
+// potential, against the pair sum: 64 x 64 x 3 8.7 us (100 us), 256 x 256 x 3
 // 18.7 us (2,056 us), 512 x 512 x 3 68 us (23.9 ms), 1024 x 1024 x 3 294 us
 // (382 ms); rel-L2 against the FP64 sum 2.5e-8 at every size, the rounding of
 // phi to FP32 (the compensated FP32 pair sum: 2e-7 .. 9e-7).  Columns are kept
 // [kx][z][y]: the column pass streams 16 Y bytes, and the four row pairs of a
 // row CTA write and read whole 128-byte lines of each column (the way back
-// with consecutive threads on consecutive pairs: 22 to 18.7 us at 256).
-struct RhoSrc {
-    const float *rho;
-    int X, Y;
-    __device__ __forceinline__ auto operator()(int z, int y) const
-    {
-        const float *r = rho + ((long long)z * Y + y) * X;
-        return [=](int x, bool) { return r[x]; };
-    }
-};
-
-template <class PL, class SRC>
-__global__ void __launch_bounds__(MAX_THREADS) k_conv_rows(ConvDev c, SRC src, double2 *__restrict__ store)
+// with consecutive threads on consecutive pairs: 22 to 18.7 us at 256).  The row
+// pass reads rho: forming the divergence of the state in it saves a launch but
+// gave each thread 48 to 96 loads, 76 us a step of 76 x 27 x 3 cells against 55.
+template <class PL>
+__global__ void __launch_bounds__(MAX_THREADS) k_conv_rows(ConvDev c, const float *__restrict__ rho,
+                                                           double2 *__restrict__ store)
 {
     extern __shared__ __align__(16) double2 cbuf[];
     pdl_begin();
-    const int np = c.Z * ((c.Y + 1) >> 1), p0 = blockIdx.x * c.fb, cs = c.cs;
-    rows_forward<row_pairs<PL>(MAX_THREADS, ROW_PAIRS)>(PL{}, c, cbuf, p0, min(c.fb, np - p0), src, [=](int k) { return store + (long long)k * cs; });
+    const int np = c.Z * ((c.Y + 1) >> 1), p0 = blockIdx.x * c.fb, cs = c.cs, X = c.X, Y = c.Y;
+    rows_forward<row_pairs<PL>(MAX_THREADS, ROW_PAIRS)>(PL{}, c, cbuf, p0, min(c.fb, np - p0),
+                                                        [=](int z, int y) {
+                                                            const float *r = rho + ((long long)z * Y + y) * X;
+                                                            return [=](int x, bool) { return r[x]; };
+                                                        },
+                                                        [=](int k) { return store + (long long)k * cs; });
 }
 
 template <class PL>
@@ -130,25 +128,29 @@ namespace mmsconv {
 
 // the shortest transform for m cells: at least 2 m - 1 long, so that no
 // wrap-around reaches a cell
-static bool fft_plan(int m, int plans, int threads, int most, FftPlan &p, int *pairs)
+static bool fft_plan(int m, bool batch, int threads, int most, FftPlan &p, int *pairs)
 {
-    for (int id = 0; id < plans; id++) {
-        with_plan(id, [&](auto pl) {
+    for (int id = 0; id < (batch ? NBATCH : NPLANS); id++) {
+        auto take = [&](auto pl) {
             using PL = decltype(pl);
             p = FftPlan{id, PL::n, PL::stride, PL::mmax};
             *pairs = row_pairs<PL>(threads, most);
-        });
+        };
+        if (batch)
+            with_batch_plan_host(id, take);
+        else
+            with_plan(id, take);
         if (p.n >= 2 * m - 1 && p.mmax <= threads) return true;
     }
     return false;
 }
 
-bool conv_layout(ConvDev &c, int X, int Y, int Z, int plans, int threads, int pairs, size_t *smem)
+bool conv_layout(ConvDev &c, int X, int Y, int Z, bool batch, int threads, int pairs, size_t *smem)
 {
     c = ConvDev{};
     int unused = 0;
-    if (X < 1 || Y < 1 || Z < 1 || Z > ZMAX || !fft_plan(X, plans, threads, pairs, c.px, &c.fb) ||
-        !fft_plan(Y, plans, threads, pairs, c.py, &unused))
+    if (X < 1 || Y < 1 || Z < 1 || Z > ZMAX || !fft_plan(X, batch, threads, pairs, c.px, &c.fb) ||
+        !fft_plan(Y, batch, threads, pairs, c.py, &unused))
         return false;
     c.X = X;
     c.Y = Y;
@@ -158,9 +160,8 @@ bool conv_layout(ConvDev &c, int X, int Y, int Z, int plans, int threads, int pa
     c.ys = (Y + 1) / 2 * 2;
     c.cs = Z * c.ys;
     c.cpg = std::max(1, threads / (Z * c.py.mmax));
-    const size_t s = std::max((size_t)c.fb * c.px.stride, (size_t)c.cpg * Z * c.py.stride) * sizeof(double2);
-    *smem = s;
-    return s <= SMEM_MAX;
+    *smem = std::max((size_t)c.fb * c.px.stride, (size_t)c.cpg * Z * c.py.stride) * sizeof(double2);
+    return *smem <= SMEM_MAX;
 }
 
 size_t conv_table_bytes(const ConvDev &c)
@@ -209,6 +210,24 @@ struct ConvPlan {
     size_t bytes = 0;
 };
 
+// layout and memory of a grid's plan: column store (first the tables'
+// scratch), tables; 0 bytes where there is none
+static size_t plan_layout(const mms_grid &g, ConvDev &c, size_t *smem, size_t *first)
+{
+    if (!conv_layout(c, g.xdim, g.ydim, g.zdim, false, MAX_THREADS, ROW_PAIRS, smem)) return 0;
+    c.cpg = 1;  // a CTA per column: the launch has few enough
+    const size_t store = (size_t)c.hx * c.cs * sizeof(double2);
+    *first = (std::max(store, conv_table_scratch(c)) + 255) / 256 * 256;
+    return *first + conv_table_bytes(c);
+}
+
+size_t conv_plan_bytes(const mms_grid &g)
+{
+    ConvDev c;
+    size_t smem = 0, first = 0;
+    return plan_layout(g, c, &smem, &first);
+}
+
 // The convolution plan of a context's grid; *out stays NULL (and MMS_OK) where
 // the pair sum serves the grid: more than ZMAX layers, rows or columns beyond
 // the transforms' length, or no memory for the column store.
@@ -217,40 +236,33 @@ int conv_plan_create(mms_ctx *ctx, ConvPlan **out)
     *out = nullptr;
     ConvPlan pl;
     ConvDev &c = pl.g;
-    size_t smem = 0;
-    if (!conv_layout(c, ctx->g.xdim, ctx->g.ydim, ctx->g.zdim, NPLANS, MAX_THREADS, ROW_PAIRS, &smem)) return MMS_OK;
-    c.cpg = 1;  // a CTA per column: the launch has few enough
-    const size_t store = (size_t)c.hx * c.cs * sizeof(double2);
-    const size_t first = (std::max(store, conv_table_scratch(c)) + 255) / 256 * 256;
-    pl.bytes = first + conv_table_bytes(c);
-    if (cudaMalloc(&pl.mem, pl.bytes) != cudaSuccess) {
-        cudaGetLastError();  // not an error of the call: the pair sum needs no store
-        return MMS_OK;
-    }
+    size_t smem = 0, first = 0;
+    pl.bytes = plan_layout(ctx->g, c, &smem, &first);
+    if (!pl.bytes || ctx_alloc(ctx, (char **)&pl.mem, pl.bytes) != MMS_OK) return MMS_OK;
     pl.store = (double2 *)pl.mem;
     int st = conv_build_tables(c, (char *)pl.mem + first, (double *)pl.mem, ctx->g.dx, ctx->g.dy, ctx->g.dz,
                                ctx->stream, &ctx->launches);
     with_plan(pl.g.px.id, [&](auto p) {
-        if (!st) st = conv_raise_smem((const void *)k_conv_rows<decltype(p), RhoSrc>, smem);
+        if (!st) st = conv_raise_smem((const void *)k_conv_rows<decltype(p)>, smem);
         if (!st) st = conv_raise_smem((const void *)k_conv_back<decltype(p)>, smem);
     });
     with_plan(pl.g.py.id, [&](auto p) {
         if (!st) st = conv_raise_smem((const void *)k_conv_columns<decltype(p)>, smem);
     });
     if (st) {
-        cudaFree(pl.mem);
+        ctx_free(ctx, pl.mem);
         return st;
     }
-    ctx->dev_bytes += pl.bytes;
     *out = new ConvPlan(pl);
     return MMS_OK;
 }
 
-void conv_plan_destroy(ConvPlan *pl)
+void conv_plan_destroy(mms_ctx *ctx)
 {
-    if (!pl) return;
-    cudaFree(pl->mem);
-    delete pl;
+    if (!ctx->conv) return;
+    ctx_free(ctx, ctx->conv->mem);
+    delete ctx->conv;
+    ctx->conv = nullptr;
 }
 
 int launch_potential_conv(mms_ctx *ctx, ConvPlan *pl, const float *rho, float *phi)
@@ -263,8 +275,7 @@ int launch_potential_conv(mms_ctx *ctx, ConvPlan *pl, const float *rho, float *p
     const size_t sc = (size_t)c.cpg * c.Z * c.py.stride * sizeof(double2);
     cudaError_t e = cudaSuccess;
     with_plan(c.px.id, [&](auto p) {
-        e = launch_k(k_conv_rows<decltype(p), RhoSrc>, dim3(div_up(pairs, c.fb)), dim3(tr), sr, ctx->stream, c,
-                     RhoSrc{rho, c.X, c.Y}, pl->store);
+        e = launch_k(k_conv_rows<decltype(p)>, dim3(div_up(pairs, c.fb)), dim3(tr), sr, ctx->stream, c, rho, pl->store);
     });
     MMS_CUDA_TRY(e);
     MMS_LAUNCH_CHECK(ctx);

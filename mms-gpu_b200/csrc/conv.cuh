@@ -48,20 +48,23 @@ struct Radices {
     static constexpr int stride = (n + (n >> shift)) | 1;  // odd: lanes on different transforms, different banks
 };
 
-constexpr int NPLANS = 19;
-
+// The lengths, in two sets of radices.  Single grids take small ones: many
+// threads with little each, so that a launch of a few CTAs ends soon (64 x 64 x 3:
+// 77 us a step against 89 with the other set).  Batches take few passes with
+// balanced radices, and stop at 512 (512 instances: 602 us a step against 710).
+constexpr int NPLANS = 19, NBATCH = 13;
 template <class F>
 void with_plan(int id, F &&f)
 {
     switch (id) {
     case 0: f(Radices<4, 4>{}); break;          // 16
     case 1: f(Radices<8, 4>{}); break;          // 32
-    case 2: f(Radices<8, 6>{}); break;          // 48
+    case 2: f(Radices<4, 4, 3>{}); break;       // 48
     case 3: f(Radices<8, 8>{}); break;          // 64
-    case 4: f(Radices<8, 10>{}); break;         // 80
-    case 5: f(Radices<8, 12>{}); break;       // 96
-    case 6: f(Radices<16, 8>{}); break;         // 128
-    case 7: f(Radices<16, 10>{}); break;       // 160
+    case 4: f(Radices<4, 5, 4>{}); break;       // 80
+    case 5: f(Radices<8, 4, 3>{}); break;       // 96
+    case 6: f(Radices<8, 4, 4>{}); break;       // 128
+    case 7: f(Radices<8, 5, 4>{}); break;       // 160
     case 8: f(Radices<8, 8, 3>{}); break;       // 192
     case 9: f(Radices<8, 8, 4>{}); break;       // 256
     case 10: f(Radices<8, 8, 5>{}); break;      // 320
@@ -76,26 +79,34 @@ void with_plan(int id, F &&f)
     }
 }
 
-// the lengths up to 512 in one kernel (the batched form: a CTA's length is its
-// instance's)
-constexpr int NBATCH = 13;
+#define MMS_CONV_BATCH_PLANS(f)                              \
+    case 0: f(Radices<4, 4>{}); break;                       \
+    case 1: f(Radices<8, 4>{}); break;                       \
+    case 2: f(Radices<8, 6>{}); break;                       \
+    case 3: f(Radices<8, 8>{}); break;                       \
+    case 4: f(Radices<8, 10>{}); break;                      \
+    case 5: f(Radices<8, 12>{}); break;                      \
+    case 6: f(Radices<16, 8>{}); break;                      \
+    case 7: f(Radices<16, 10>{}); break;                     \
+    case 8: f(Radices<8, 8, 3>{}); break;                    \
+    case 9: f(Radices<8, 8, 4>{}); break;                    \
+    case 10: f(Radices<8, 8, 5>{}); break;                   \
+    case 11: f(Radices<16, 8, 3>{}); break;                  \
+    case 12: f(Radices<8, 8, 8>{}); break;
+
+template <class F>
+void with_batch_plan_host(int id, F &&f)
+{
+    switch (id) {
+        MMS_CONV_BATCH_PLANS(f)
+    }
+}
+// in one kernel: a CTA's length is its instance's
 template <class F>
 __device__ __forceinline__ void with_batch_plan(int id, F &&f)
 {
     switch (id) {
-    case 0: f(Radices<4, 4>{}); break;
-    case 1: f(Radices<8, 4>{}); break;
-    case 2: f(Radices<8, 6>{}); break;
-    case 3: f(Radices<8, 8>{}); break;
-    case 4: f(Radices<8, 10>{}); break;
-    case 5: f(Radices<8, 12>{}); break;
-    case 6: f(Radices<16, 8>{}); break;
-    case 7: f(Radices<16, 10>{}); break;
-    case 8: f(Radices<8, 8, 3>{}); break;
-    case 9: f(Radices<8, 8, 4>{}); break;
-    case 10: f(Radices<8, 8, 5>{}); break;
-    case 11: f(Radices<16, 8, 3>{}); break;
-    case 12: f(Radices<8, 8, 8>{}); break;
+        MMS_CONV_BATCH_PLANS(f)
     }
 }
 
@@ -300,9 +311,10 @@ __host__ __device__ __forceinline__ void dft_padded(double2 *v)
 }
 
 // host side (conv.cu)
-// dims, plans and layout of a grid for CTAs of `threads` (at most `pairs` row
-// pairs) and the first `plans` lengths; false where it has none.  *smem: what a row or column CTA needs.
-bool conv_layout(ConvDev &c, int X, int Y, int Z, int plans, int threads, int pairs, size_t *smem);
+// dims, plans and layout of a grid (batch: with the batches' radices) for CTAs
+// of `threads` with at most `pairs` row pairs; false where it has none.  *smem:
+// what a row or column CTA needs.
+bool conv_layout(ConvDev &c, int X, int Y, int Z, bool batch, int threads, int pairs, size_t *smem);
 // bytes of the twiddles and Ghat for these lengths and layers, and of the
 // scratch their construction needs
 size_t conv_table_bytes(const ConvDev &c);

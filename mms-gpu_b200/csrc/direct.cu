@@ -1,11 +1,11 @@
 // Exact demag potential: phi_i = sum_{j != i} rho_j dV / |r_i - r_j| (the
 // reference's calc_potential_exact, fmm_calc.cu:412-461, and its GPU kernel
 // potential_calc.cu:18-116).  Contexts evaluate it as a convolution (conv.cu)
-// where the grid has a plan; this file is the O(N^2) pair sum, for the other
-// grids (PAIR_CELLS_MAX, more than 8 layers, rows or columns beyond the
-// transforms) and for the allocation-free entry point.
+// where the grid has a plan, small grids in one launch (k_direct_small); the
+// O(N^2) pair sum k_direct is for the other grids (more than 8 layers, rows or
+// columns beyond the transforms) and for the allocation-free entry point.
 //
-// B200 design of the pair sum.  On a regular grid 1/|r_i - r_j| depends only on the integer
+// B200 design of k_direct.  On a regular grid 1/|r_i - r_j| depends only on the integer
 // offset, so the sum is a 3-D aperiodic convolution.  A table
 // G[|dz|][|dy|][|dx|] = dV/|r| is built once per context in FP64 and rounded to
 // FP32 (more accurate than a per-pair rsqrt, and it takes the MUFU pipe out of
@@ -26,9 +26,14 @@
 //     groups (the long reduction), each group's row product (one FP32 FMA chain
 //     per target) being a plain FP32 partial; the warps' partials are combined in FP64 in a fixed
 //     order, so results are bitwise reproducible run to run.
+#include "conv.cuh"
 #include "mms_internal.cuh"
+#include "stencil_dev.cuh"
+#include "umma.cuh"
 
 #include <math.h>
+
+#include <algorithm>
 
 #include <mutex>
 
@@ -38,11 +43,6 @@ constexpr int TX = 8;            // targets per lane
 constexpr int SEG = 32 * TX;     // targets per warp segment
 constexpr int DWARPS = 4;        // warps per CTA splitting the groups of a row
 constexpr int MAX_X = 2048;      // row length limit of the shared-memory staging
-// Grids of at most this many cells take the pair sum: one launch against the
-// convolution's three.  8 x 8 x 3: 9.2 us a call against 13.3; 16 x 16 x 3:
-// 16.5 against 13.4 (back-to-back calls).
-constexpr long long PAIR_CELLS_MAX = 256;
-
 __global__ void k_build_gtab(float *__restrict__ gtab, GridK g)
 {
     long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -199,7 +199,164 @@ size_t direct_smem_bytes(int X)
     return (size_t)DWARPS * (sh.Xr + sh.GM) * sizeof(float) + (size_t)DWARPS * SEG * 2 * sizeof(float);
 }
 
+// ---- small grids: the whole sum in one launch --------------------------------
+// CTA = a segment of one target row.  It stages the mirrored table and every
+// charge of the grid (formed from M where that is given) in shared memory; a
+// thread holds 4 consecutive targets and takes every S-th source row, 16 FMAs
+// per two 16-byte reads as in k_direct; a row's FP32 sum is added to FP64 sums,
+// and the S partial sums of a target are added in a fixed order.
+constexpr int SMALL_THREADS = 512;
+constexpr size_t SMALL_SMEM = 200 * 1024;
+
+struct SmallShape {
+    int X, Y, Z, rows;   // rows = Y Z
+    int Xr, C, pitch;    // row of charges, centre and length of a mirrored row (floats)
+    int segs, tiles, S;  // segments a row, threads' tiles of 4 targets a segment, source-row splits
+};
+
+// gm[|dz|][|dy|][C + dx] = dV/|r|, 0 beyond the grid and at the origin
+__global__ void k_build_gsmall(float *__restrict__ gm, SmallShape s, double dx, double dy, double dz)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= s.rows * s.pitch) return;
+    const int d = abs(i % s.pitch - s.C), y = i / s.pitch % s.Y, z = i / s.pitch / s.Y;
+    const double rx = d * dx, ry = y * dy, rz = z * dz, r2 = rx * rx + ry * ry + rz * rz;
+    gm[i] = d >= s.X || r2 == 0.0 ? 0.f : (float)(dx * dy * dz / sqrt(r2));
+}
+
+template <int SRC>  // 0: rho, 1: FP64 state, 2: FP32 M
+__global__ void __launch_bounds__(SMALL_THREADS) k_direct_small(ChargeSrc src, const float *__restrict__ gtab,
+                                                                float *__restrict__ phi, SmallShape s, GridK g,
+                                                                mmsdev::DivScale h, mmsdev::DivAos d)
+{
+    extern __shared__ __align__(16) float sm[];
+    float *gm = sm, *qs = gm + s.rows * s.pitch;
+    double *red = reinterpret_cast<double *>(qs + s.rows * s.Xr);  // [S][4 tiles]
+    __shared__ int nz[SMALL_THREADS];  // source row holds charge (rows <= SMALL_THREADS)
+    for (int i = threadIdx.x * 4; i < s.rows * s.pitch; i += blockDim.x * 4)
+        umma::cp_async16(umma::smem_u32(gm + i), gtab + i, true);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    for (int i = threadIdx.x; i < s.rows; i += blockDim.x) nz[i] = 0;
+    __syncthreads();
+    pdl_begin();  // the table is constant; the charges are the predecessor's output
+    const int trow = blockIdx.x / s.segs, seg = blockIdx.x % s.segs;
+    constexpr int U = 4;  // cells a thread has in flight
+    for (int e0 = threadIdx.x; e0 < s.rows * s.Xr; e0 += U * blockDim.x) {
+        float v[U];
+        int row[U];
+        bool in[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int e = min(e0 + u * (int)blockDim.x, s.rows * s.Xr - 1);
+            row[u] = e / s.Xr;
+            const int x = min(e - row[u] * s.Xr, s.X - 1), z = row[u] / s.Y, y = row[u] - z * s.Y;
+            in[u] = e - row[u] * s.Xr < s.X;
+            const int i = row[u] * s.X + x;
+            if (SRC == 1)
+                v[u] = mmsdev::div_soa_cell<true>(src.M, i, x, y, z, g, h);
+            else if (SRC == 2)
+                v[u] = mmsdev::div_aos_cell(src.Ma, i, x, y, z, g, d);
+            else
+                v[u] = src.rho[i];
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int e = e0 + u * blockDim.x;
+            if (e >= s.rows * s.Xr) break;
+            qs[e] = in[u] ? v[u] : 0.f;
+            if (in[u] && v[u] != 0.f) nz[row[u]] = 1;  // any writer stores 1
+            if (SRC == 2 && src.charge && in[u] && seg == 0 && row[u] == trow)
+                src.charge[row[u] * s.X + e - row[u] * s.Xr] = v[u];
+        }
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+    const int yt = trow % s.Y, zt = trow / s.Y;
+    const int tile = threadIdx.x % s.tiles, split = threadIdx.x / s.tiles;
+    const int x0 = 4 * (seg * s.tiles + tile);
+    if (split < s.S && x0 < s.Xr) {
+        double tot[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int r = split; r < s.rows; r += s.S) {
+            if (!nz[r]) continue;
+            const int zs = r / s.Y, ys = r - zs * s.Y;
+            const float *grow = gm + (abs(zt - zs) * s.Y + abs(yt - ys)) * s.pitch;
+            const float4 *q4 = reinterpret_cast<const float4 *>(qs + r * s.Xr);
+            float acc[4] = {0.f, 0.f, 0.f, 0.f};
+            // window win[k] = grow[base + k], base = C - 3 + x0 - xs
+            const float4 *w4 = reinterpret_cast<const float4 *>(grow + s.C - 3 + x0);
+            float4 b = w4[1];
+#pragma unroll 4
+            for (int t = 0; t < s.Xr / 4; t++) {
+                const float4 a = w4[-t], q = q4[t];
+                const float win[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}, qv[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+#pragma unroll
+                    for (int i = 0; i < 4; i++) acc[i] = fmaf(qv[j], win[3 + i - j], acc[i]);
+                b = a;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) tot[i] += (double)acc[i];
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) red[split * 4 * s.tiles + 4 * tile + i] = tot[i];
+    }
+    __syncthreads();
+    for (int o = threadIdx.x; o < 4 * s.tiles; o += blockDim.x) {
+        const int x = 4 * seg * s.tiles + o;
+        if (x >= s.X) break;
+        double t = 0.0;
+#pragma unroll 8
+        for (int k = 0; k < s.S; k++) t += red[k * 4 * s.tiles + o];
+        phi[trow * s.X + x] = (float)t;
+    }
+}
+
+size_t small_smem(const SmallShape &s)
+{
+    return ((size_t)s.rows * (s.pitch + s.Xr)) * sizeof(float) + (size_t)s.S * 4 * s.tiles * sizeof(double);
+}
+
+// Where the one-launch sum serves.  A call of its own (potential, field) is
+// bound by its launches: 16 x 16 x 3 5.0 us against 11.9 for the convolution's
+// three, 40 x 40 x 3 9.4 against 12.0, 76 x 27 x 3 11.7 against 12.1.  In a
+// captured step the launches cost less and every CTA's pass over all charges
+// more: 16 x 16 x 3 39 us a step against 41, 24 x 24 x 3 49 against 44,
+// 40 x 40 x 3 78 against 51.
+constexpr long long SMALL_CALL_MAX = 5000, SMALL_STEP_MAX = 1024;
+bool small_shape(const mms_grid &g, SmallShape &s)
+{
+    if ((long long)g.xdim * g.ydim * g.zdim > SMALL_CALL_MAX || g.ydim * g.zdim > SMALL_THREADS) return false;
+    s.X = g.xdim;
+    s.Y = g.ydim;
+    s.Z = g.zdim;
+    s.rows = s.Y * s.Z;
+    s.Xr = (s.X + 3) & ~3;
+    s.C = s.Xr + 3;
+    s.pitch = 2 * s.Xr + 8;
+    // two CTAs an SM at most, whole tiles a segment, every thread a source row
+    const int all = s.Xr / 4;
+    s.segs = std::max(1, std::min(all, 296 / s.rows));
+    s.tiles = (all + s.segs - 1) / s.segs;
+    s.segs = (all + s.tiles - 1) / s.tiles;
+    s.S = std::max(1, std::min(s.rows, SMALL_THREADS / s.tiles));
+    return s.tiles <= SMALL_THREADS && small_smem(s) <= SMALL_SMEM;
+}
+
 }  // namespace
+
+size_t direct_bytes(const mms_grid &g)
+{
+    const size_t N = (size_t)g.xdim * g.ydim * g.zdim;
+    SmallShape s;
+    size_t b = 0;
+    if (small_shape(g, s)) {
+        b = ((size_t)s.rows * s.pitch * sizeof(float) + 255) / 256 * 256;
+        if (N <= SMALL_STEP_MAX) return b;
+    }
+    const size_t c = conv_plan_bytes(g);
+    return b + (c ? (c + 255) / 256 * 256 : (N * sizeof(float) + 255) / 256 * 256);
+}
 
 int direct_prepare(mms_ctx *ctx)
 {
@@ -207,8 +364,19 @@ int direct_prepare(mms_ctx *ctx)
         mms_set_error("direct sum: xdim %d exceeds the supported %d", ctx->g.xdim, MAX_X);
         return MMS_ERR_ARG;
     }
-    if (ctx->conv || ctx->gtab) return MMS_OK;
-    if (ctx->N > PAIR_CELLS_MAX) MMS_TRY(conv_plan_create(ctx, &ctx->conv));
+    if (ctx->conv || ctx->gtab || (ctx->gsmall && ctx->N <= SMALL_STEP_MAX)) return MMS_OK;
+    SmallShape s;
+    if (!ctx->gsmall && small_shape(ctx->g, s)) {
+        MMS_TRY(ctx_alloc(ctx, &ctx->gsmall, (size_t)s.rows * s.pitch));
+        k_build_gsmall<<<div_up((long long)s.rows * s.pitch, 256), 256, 0, ctx->stream>>>(ctx->gsmall, s, ctx->g.dx,
+                                                                                      ctx->g.dy, ctx->g.dz);
+        MMS_LAUNCH_CHECK(ctx);
+        MMS_TRY(mmsconv::conv_raise_smem((const void *)k_direct_small<0>, SMALL_SMEM));
+        MMS_TRY(mmsconv::conv_raise_smem((const void *)k_direct_small<1>, SMALL_SMEM));
+        MMS_TRY(mmsconv::conv_raise_smem((const void *)k_direct_small<2>, SMALL_SMEM));
+        if (ctx->N <= SMALL_STEP_MAX) return MMS_OK;
+    }
+    MMS_TRY(conv_plan_create(ctx, &ctx->conv));
     if (ctx->conv) return MMS_OK;
     MMS_TRY(ctx_alloc(ctx, &ctx->gtab, (size_t)ctx->N));
     k_build_gtab<<<div_up(ctx->N, 256), 256, 0, ctx->stream>>>(ctx->gtab, ctx->gk());
@@ -222,15 +390,59 @@ int direct_prepare(mms_ctx *ctx)
     return MMS_OK;
 }
 
+namespace {
+
+int launch_small(mms_ctx *ctx, const ChargeSrc &src, float *phi)
+{
+    SmallShape s;
+    small_shape(ctx->g, s);
+    auto kern = src.M ? k_direct_small<1> : src.Ma ? k_direct_small<2> : k_direct_small<0>;
+    const int threads = std::max(128, (s.S * s.tiles + 31) / 32 * 32);
+    MMS_CUDA_TRY(launch_k(kern, dim3((unsigned)(s.rows * s.segs)), dim3((unsigned)threads), small_smem(s), ctx->stream,
+                          src, (const float *)ctx->gsmall, phi, s, ctx->gk(),
+                          mmsdev::div_scale(ctx->g.dx, ctx->g.dy, ctx->g.dz),
+                          mmsdev::DivAos{(float)ctx->g.dx, (float)ctx->g.dy, (float)ctx->g.dz}));
+    MMS_LAUNCH_CHECK(ctx);
+    return MMS_OK;
+}
+
+}  // namespace
+
 int launch_potential_direct(mms_ctx *ctx, const float *rho, float *phi)
 {
     MmsRange nvtx_("mms/direct_potential");
     MMS_TRY(direct_prepare(ctx));
+    ChargeSrc src;
+    src.rho = rho;
+    if (ctx->gsmall) return launch_small(ctx, src, phi);
     if (ctx->conv) return launch_potential_conv(ctx, ctx->conv, rho, phi);
     dim3 grid((unsigned)(ctx->g.ydim * ctx->g.zdim), div_up(ctx->g.xdim, SEG));
     k_direct<<<grid, DWARPS * 32, direct_smem_bytes(ctx->g.xdim), ctx->stream>>>(rho, ctx->gtab, phi, ctx->gk());
     MMS_LAUNCH_CHECK(ctx);
     return MMS_OK;
+}
+
+int launch_potential_direct_state(mms_ctx *ctx, const double *M, float *phi)
+{
+    MMS_TRY(direct_prepare(ctx));
+    ChargeSrc src;
+    src.M = M;
+    if (ctx->gsmall && ctx->N <= SMALL_STEP_MAX) return launch_small(ctx, src, phi);
+    MMS_TRY(launch_divergence_soa(ctx, M, ctx->rho));
+    if (ctx->conv) return launch_potential_conv(ctx, ctx->conv, ctx->rho, phi);
+    return launch_potential_direct(ctx, ctx->rho, phi);
+}
+
+int launch_potential_direct_aos(mms_ctx *ctx, const float *M, float *charge, float *phi)
+{
+    MMS_TRY(direct_prepare(ctx));
+    ChargeSrc src;
+    src.Ma = M;
+    src.charge = charge;
+    if (ctx->gsmall) return launch_small(ctx, src, phi);
+    float *rho = charge ? charge : ctx->rho;
+    MMS_TRY(launch_divergence_aos(ctx, M, rho));
+    return launch_potential_direct(ctx, rho, phi);
 }
 
 // ---------------------------------------------------------------------------

@@ -655,7 +655,7 @@ int ens_conv_prepare(mms_ens *e)
     for (int i = 0; i < e->n; i++) {
         ConvDev &c = conv[i].c;
         size_t s = 0;
-        if (!conv_layout(c, e->hin[i].X, e->hin[i].Y, e->hin[i].Z, NBATCH, CONV_THREADS, CONV_PAIRS, &s))
+        if (!conv_layout(c, e->hin[i].X, e->hin[i].Y, e->hin[i].Z, true, CONV_THREADS, CONV_PAIRS, &s))
             return MMS_OK;
         smem = std::max(smem, s);
         conv[i].off = e->hin[i].off;

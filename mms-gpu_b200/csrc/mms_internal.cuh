@@ -116,11 +116,17 @@ struct mms_ctx {
     int64_t launches = 0;
     size_t dev_bytes = 0;
 
+    // one allocation for the buffers below and the exact potential's tables:
+    // 17 of their own took 3.3 ms to map at 256 x 256 x 3
+    char *arena = nullptr;
+    size_t arena_bytes = 0, arena_used = 0;
+
     // device buffers
     float *rho = nullptr, *phi = nullptr;       // N
     float *vecA = nullptr, *vecB = nullptr;     // 3N FP32 AoS scratch (host API)
     ConvPlan *conv = nullptr;                   // exact potential as a convolution
     float *gtab = nullptr;                      // pair-sum kernel table X*Y*Z, where there is no convolution plan
+    float *gsmall = nullptr;                    // mirrored table of the one-launch sum (small grids)
     uint8_t *mat = nullptr;                     // N
     double *M = nullptr, *A = nullptr, *B = nullptr, *K = nullptr;  // 3N each, SoA planes
     double *Mbak = nullptr;                     // 3N, controller backup
@@ -174,12 +180,25 @@ int launch_hfield_aos(mms_ctx *ctx, const float *M, const float *phi, double t, 
 int launch_rk4_stage(mms_ctx *ctx, int stage, const double *Mst, double *Mnext);
 int launch_stats(mms_ctx *ctx);
 
+// where the charges of an exact potential come from
+struct ChargeSrc {
+    const float *rho = nullptr;   // given,
+    const double *M = nullptr;    // or the divergence of the FP64 state,
+    const float *Ma = nullptr;    // or of FP32 M,
+    float *charge = nullptr;      // stored here unless NULL
+};
 // exact potential: the convolution where the grid has a plan, else the pair sum
 int direct_prepare(mms_ctx *ctx);
+size_t direct_bytes(const mms_grid &g);  // device memory of its tables and store
 int conv_plan_create(mms_ctx *ctx, ConvPlan **out);
-void conv_plan_destroy(ConvPlan *pl);
+size_t conv_plan_bytes(const mms_grid &g);
+void conv_plan_destroy(mms_ctx *ctx);
 int launch_potential_conv(mms_ctx *ctx, ConvPlan *pl, const float *rho, float *phi);
 int launch_potential_direct(mms_ctx *ctx, const float *rho, float *phi);
+// the same with rho = div M formed on the way: of the FP64 state M, or of FP32
+// M (N x 3) with the reference's bits, stored to `charge` unless that is NULL
+int launch_potential_direct_state(mms_ctx *ctx, const double *M, float *phi);
+int launch_potential_direct_aos(mms_ctx *ctx, const float *M, float *charge, float *phi);
 
 int fmm_plan_create(mms_ctx *ctx);
 int launch_potential_surrogate(mms_ctx *ctx, const float *rho, float *phi);
@@ -254,20 +273,34 @@ cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sme
     return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-// device allocation tracked in ctx->dev_bytes
+// device allocation tracked in ctx->dev_bytes: from the context's arena while
+// it has room, else its own (ctx_free knows which)
 template <class T>
 int ctx_alloc(mms_ctx *ctx, T **p, size_t count)
 {
     size_t bytes = count * sizeof(T);
     if (bytes == 0) bytes = 16;
+    const size_t padded = (bytes + 255) / 256 * 256;
+    if (ctx->arena && ctx->arena_used + padded <= ctx->arena_bytes) {
+        *p = (T *)(ctx->arena + ctx->arena_used);
+        ctx->arena_used += padded;
+        ctx->dev_bytes += bytes;
+        return MMS_OK;
+    }
     cudaError_t e = cudaMalloc((void **)p, bytes);
     if (e != cudaSuccess) {
+        cudaGetLastError();  // reported here; not to be found pending by a later call
         *p = nullptr;
         mms_set_error("cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
         return MMS_ERR_NOMEM;
     }
     ctx->dev_bytes += bytes;
     return MMS_OK;
+}
+
+inline void ctx_free(mms_ctx *ctx, void *p)
+{
+    if (p && !(ctx->arena && (char *)p >= ctx->arena && (char *)p < ctx->arena + ctx->arena_bytes)) cudaFree(p);
 }
 
 static inline unsigned div_up(long long a, long long b) { return (unsigned)((a + b - 1) / b); }

@@ -35,16 +35,7 @@ __global__ void k_div_aos(const float *__restrict__ M, float *__restrict__ rho, 
     if (i >= g.N) return;
     int x, y, z;
     cell_xyz(i, g, x, y, z);
-    const long long sx = 1, sy = g.X, sz = (long long)g.X * g.Y;
-    float x2 = (x != g.X - 1) ? M[3 * (i + sx) + 0] : 0.f;
-    float x0 = (x != 0) ? M[3 * (i - sx) + 0] : 0.f;
-    float y2 = (y != g.Y - 1) ? M[3 * (i + sy) + 1] : 0.f;
-    float y0 = (y != 0) ? M[3 * (i - sy) + 1] : 0.f;
-    float z2 = (z != g.Z - 1) ? M[3 * (i + sz) + 2] : 0.f;
-    float z0 = (z != 0) ? M[3 * (i - sz) + 2] : 0.f;
-    float s = __fadd_rn(__fadd_rn(__fdiv_rn(__fsub_rn(x2, x0), dx), __fdiv_rn(__fsub_rn(y2, y0), dy)),
-                        __fdiv_rn(__fsub_rn(z2, z0), dz));
-    rho[i] = s * 0.5f;  // (s / 2.0) in double then to float: exact halving
+    rho[i] = div_aos_cell(M, i, x, y, z, g, DivAos{dx, dy, dz});
 }
 
 // vector_functions.cpp:31-54; c is the reference's fptype constant_multiple

@@ -201,9 +201,9 @@ int autotune(const mms_grid *grid, const mms_params *params, const float *rho_de
     } while (0);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
-    if (exact) cudaFree(exact);
-    if (phi) cudaFree(phi);
-    if (part) cudaFree(part);
+    ctx_free(ctx, exact);
+    ctx_free(ctx, phi);
+    ctx_free(ctx, part);
     mms_ctx_destroy(ctx);
     if (st != MMS_OK) return st;
     if (!found) {
