@@ -2,6 +2,7 @@
 // FP64 RK4 state, the fixed-step driver (optionally one CUDA graph per step)
 // and the adaptive marching loop.
 #include "mms_internal.cuh"
+#include "stencil_dev.cuh"
 
 #include <math.h>
 #include <stdarg.h>
@@ -25,8 +26,15 @@ namespace {
 
 __global__ void k_set_dt(double *tstate, double dt) { tstate[TIME_DT] = dt; }
 
-__global__ void k_set_time(double *tstate, double t, double tk1, double dt)
+// new parameters: H_ext of the next step's first stage
+__global__ void k_set_hext(double *tstate, const double *htab, PhysK p)
 {
+    mmsdev::put_hext(p, htab, tstate, 0, tstate[p.ref_stage_time ? TIME_TK1 : TIME_T]);
+}
+
+__global__ void k_set_time(double *tstate, double t, double tk1, double dt, const double *htab, PhysK p)
+{
+    mmsdev::put_hext(p, htab, tstate, 0, p.ref_stage_time ? tk1 : t);
     tstate[TIME_T] = t;
     tstate[TIME_TK1] = tk1;
     tstate[TIME_DT] = dt;
@@ -39,10 +47,12 @@ __global__ void k_set_time(double *tstate, double t, double tk1, double dt)
 // cleared
 template <typename T>
 __global__ void k_state_in(const T *__restrict__ in, const uint8_t *mat_in, uint8_t *mat, double *__restrict__ out,
-                           long long N, double *__restrict__ tstate, double *__restrict__ stats, double t)
+                           long long N, double *__restrict__ tstate, double *__restrict__ stats, double t,
+                           const double *__restrict__ htab, PhysK p)
 {
     long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i == 0) {
+        mmsdev::put_hext(p, htab, tstate, 0, t);
         tstate[TIME_T] = t;
         tstate[TIME_TK1] = t;
         tstate[TIME_DT] = 0.0;
@@ -152,6 +162,8 @@ int apply_params(mms_ctx *ctx, const mms_params *p)
     }
     MMS_CUDA_TRY(cudaMemcpyAsync(ctx->hext, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice,
                                  ctx->stream));
+    k_set_hext<<<1, 1, 0, ctx->stream>>>(ctx->tstate, ctx->hext, ctx->pk());
+    MMS_LAUNCH_CHECK(ctx);
     MMS_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     return MMS_OK;
 }
@@ -634,7 +646,7 @@ int mms_state_set_dev(mms_ctx *ctx, const uint8_t *material, const double *M, do
         return MMS_ERR_ARG;
     }
     k_state_in<double><<<div_up(ctx->N, 256), 256, 0, ctx->stream>>>(M, material, ctx->mat, ctx->M, ctx->N,
-                                                                     ctx->tstate, ctx->stats, t);
+                                                                     ctx->tstate, ctx->stats, t, ctx->hext, ctx->pk());
     MMS_LAUNCH_CHECK(ctx);
     ctx->dt_known = false;
     ctx->state_ready = true;
@@ -652,7 +664,7 @@ int mms_state_set(mms_ctx *ctx, const uint8_t *material, const double *M, double
     MMS_CUDA_TRY(cudaMemcpyAsync(ctx->mat, material, n, cudaMemcpyHostToDevice, ctx->stream));
     MMS_CUDA_TRY(cudaMemcpyAsync(ctx->K, M, 3 * n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     k_state_in<double><<<div_up(ctx->N, 256), 256, 0, ctx->stream>>>(ctx->K, ctx->mat, ctx->mat, ctx->M, ctx->N,
-                                                                     ctx->tstate, ctx->stats, t);
+                                                                     ctx->tstate, ctx->stats, t, ctx->hext, ctx->pk());
     MMS_LAUNCH_CHECK(ctx);
     ctx->dt_known = false;
     MMS_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
@@ -705,7 +717,7 @@ int mms_state_set_f32_dev(mms_ctx *ctx, const uint8_t *material, const float *M,
         return MMS_ERR_ARG;
     }
     k_state_in<float><<<div_up(ctx->N, 256), 256, 0, ctx->stream>>>(M, material, ctx->mat, ctx->M, ctx->N,
-                                                                    ctx->tstate, ctx->stats, t);
+                                                                    ctx->tstate, ctx->stats, t, ctx->hext, ctx->pk());
     MMS_LAUNCH_CHECK(ctx);
     ctx->dt_known = false;
     ctx->state_ready = true;
@@ -739,7 +751,7 @@ int mms_state_set_f32(mms_ctx *ctx, const uint8_t *material, const float *M, dou
     MMS_CUDA_TRY(cudaMemcpyAsync(ctx->mat, material, n, cudaMemcpyHostToDevice, ctx->stream));
     MMS_CUDA_TRY(cudaMemcpyAsync(stage, M, 3 * n * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     k_state_in<float><<<div_up(ctx->N, 256), 256, 0, ctx->stream>>>(stage, ctx->mat, ctx->mat, ctx->M, ctx->N,
-                                                                    ctx->tstate, ctx->stats, t);
+                                                                    ctx->tstate, ctx->stats, t, ctx->hext, ctx->pk());
     MMS_LAUNCH_CHECK(ctx);
     ctx->dt_known = false;
     MMS_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
@@ -855,7 +867,7 @@ int mms_march(mms_ctx *ctx, const mms_controller *ctl, double finaltime, double 
         MMS_CUDA_TRY(cudaMemcpyAsync(ctx->M, ctx->Mbak, n3 * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
         MMS_CUDA_TRY(cudaMemcpyAsync(ctx->phi, ctx->phibak, (size_t)ctx->N * sizeof(float), cudaMemcpyDeviceToDevice,
                                      ctx->stream));
-        k_set_time<<<1, 1, 0, ctx->stream>>>(ctx->tstate, t_, tk1_, 0.0);
+        k_set_time<<<1, 1, 0, ctx->stream>>>(ctx->tstate, t_, tk1_, 0.0, ctx->hext, ctx->pk());
         MMS_LAUNCH_CHECK(ctx);
         ctx->dt_known = false;
         ctx->phi_valid = true;

@@ -825,7 +825,7 @@ int mms_ens_create(const mms_ens_instance *inst, int n, double dx, double dy, do
         if ((st = ens_alloc(e, &e->K, 3 * N))) break;
         if ((st = ens_alloc(e, &e->tstate, TIME_SLOTS))) break;
         if ((st = ens_alloc(e, &e->flag, 1))) break;
-        if (cudaMallocHost((void **)&e->h_scratch, 8 * sizeof(double)) != cudaSuccess) {
+        if (cudaMallocHost((void **)&e->h_scratch, (TIME_SLOTS + 4) * sizeof(double)) != cudaSuccess) {
             st = MMS_ERR_NOMEM;
             mms_set_error("cudaMallocHost failed");
             break;

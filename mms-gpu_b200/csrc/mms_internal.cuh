@@ -92,10 +92,13 @@ inline void physk_derive(PhysK &k, double dx, double dy, double dz)
 //   [1] dt     step size
 //   [2] t_k1   time at which H(M) (the k1 field) was evaluated; equals t
 //              except in reference-stage-time mode (see mms_params)
-constexpr int TIME_T = 0, TIME_DT = 1, TIME_TK1 = 2, TIME_SLOTS = 4;
+constexpr int TIME_T = 0, TIME_DT = 1, TIME_TK1 = 2;
 //   [3] (low 32 bits) arrival counter of the last RK4 stage's CTAs: the last
 //       to finish advances the time and resets it (k_rk4_stage)
 constexpr int TIME_CTR = 3;
+//   [4 + 3 s ..] H_ext at the time of RK4 stage s where a table is given:
+//       formed while the stage before it runs (put_hext)
+constexpr int TIME_HEXT = 4, TIME_SLOTS = 16;
 
 // statistics block: sums over material cells, finished on device
 //   [0] sum M.H  [1] max |MxH|  [2..4] sum M  [5] sum |M|  [6] count  [7] nonfinite flag

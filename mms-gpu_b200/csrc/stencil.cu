@@ -162,6 +162,7 @@ __global__ void k_div_soa(const double *__restrict__ M, float *__restrict__ rho,
 //   stage 2: K += 2 k3;     Mnext = M + dt   k3
 //   stage 3: K += k4;       M = renorm(M + dt/6 K) (Mnext unused, written in place)
 // Empty cells keep M = 0 in every buffer.
+template <bool TAB, bool EAGER>
 __device__ __forceinline__ void rk4_stage_cell(long long i, const float *__restrict__ phi,
                                                const double *__restrict__ Mst, double *__restrict__ M,
                                                double *__restrict__ K, double *__restrict__ Mnext,
@@ -171,33 +172,34 @@ __device__ __forceinline__ void rk4_stage_cell(long long i, const float *__restr
 {
     const long long N = g.N;
     const double t = tstate[TIME_T], dt = tstate[TIME_DT];
-    if (!mat[i]) {
-        if (stage < 3) {
-            Mnext[i] = 0.0;
-            Mnext[i + N] = 0.0;
-            Mnext[i + 2 * N] = 0.0;
-        } else {
-            M[i] = 0.0;
-            M[i + N] = 0.0;
-            M[i + 2 * N] = 0.0;
-        }
+    double he[3];
+    if (TAB)
+        for (int c = 0; c < 3; c++) he[c] = tstate[TIME_HEXT + 3 * stage + c];
+    double *const out = stage < 3 ? Mnext : M;
+    if (!EAGER && !mat[i]) {
+        for (int c = 0; c < 3; c++) out[i + c * N] = 0.0;
         return;
     }
     int x, y, z;
     cell_xyz(i, g, x, y, z);
-    double ts;
-    if (p.ref_stage_time)
-        ts = (stage == 0) ? tstate[TIME_TK1] : t;
-    else
-        ts = t + ((stage == 0) ? 0.0 : (stage == 3 ? dt : 0.5 * dt));
-    double he[3];
-    hext_at(p, htab, ts, he);
+    if (!TAB) {
+        double ts;
+        if (p.ref_stage_time)
+            ts = (stage == 0) ? tstate[TIME_TK1] : t;
+        else
+            ts = t + ((stage == 0) ? 0.0 : (stage == 3 ? dt : 0.5 * dt));
+        hext_at(p, htab, ts, he);
+    }
     double h[3];
-    field_soa(phi, Mst, i, x, y, z, g, p, he, h);
+    field_soa<TAB>(phi, Mst, i, x, y, z, g, p, he, h);
     const double ms[3] = {Mst[i], Mst[i + N], Mst[i + 2 * N]};
     double k[3];
     llg(ms, h, p, k);
     const double m[3] = {M[i], M[i + N], M[i + 2 * N]};
+    if (EAGER && !mat[i]) {
+        for (int c = 0; c < 3; c++) out[i + c * N] = 0.0;
+        return;
+    }
     if (stage == 0) {
         K[i] = k[0];
         K[i + N] = k[1];
@@ -233,6 +235,18 @@ __device__ __forceinline__ void rk4_stage_cell(long long i, const float *__restr
 // last CTA to finish also advances the time of the state, so that no launch
 // of its own follows the step: every CTA has read t and dt before it arrives
 // on the counter, and the counter is reset for the next step.
+//
+// Bound by the latency of its dependent loads: time, table search, mask,
+// neighbours.  TAB (an external-field table is given): a CTA of its own forms
+// H_ext for the stage after this one (put_hext), so that a cell reads it like
+// any operand, and the neighbours' loads are unconditional: 76 x 27 x 3 exact
+// steps 57.6 -> 54.9 us, 64 x 64 x 3 FMM 119.0 -> 117.0, 256 x 256 x 3 FMM
+// 135.7 -> 134.0.  Without a table there is no search to save, and the same
+// code measured 0 to 2 us a step slower.  EAGER (to two CTAs an SM): the loads
+// do not wait for the mask either: 54.9 -> 53.8 and 117.0 -> 115.5 us; at 256 x
+// 256 x 3, where the loads of empty cells cost bandwidth, 134.0 -> 136.9.
+constexpr long long EAGER_MAX = 2 * 148 * TPB;
+template <bool TAB, bool EAGER>
 __global__ void __launch_bounds__(TPB) k_rk4_stage(const float *__restrict__ phi, const double *__restrict__ Mst,
                                                    double *__restrict__ M, double *__restrict__ K,
                                                    double *__restrict__ Mnext, const uint8_t *__restrict__ mat,
@@ -241,8 +255,14 @@ __global__ void __launch_bounds__(TPB) k_rk4_stage(const float *__restrict__ phi
                                                    int advance)
 {
     pdl_begin();
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i < g.N) rk4_stage_cell(i, phi, Mst, M, K, Mnext, mat, tstate, htab, stats, g, p, stage);
+    const long long i = (blockIdx.x - (TAB ? 1u : 0u)) * (long long)blockDim.x + threadIdx.x;
+    if (!TAB || blockIdx.x > 0) {
+        if (i < g.N) rk4_stage_cell<TAB, EAGER>(i, phi, Mst, M, K, Mnext, mat, tstate, htab, stats, g, p, stage);
+    } else if (threadIdx.x == 0) {
+        const double t = tstate[TIME_T], dt = tstate[TIME_DT];
+        const double ahead = p.ref_stage_time ? 0.0 : (stage < 2 ? 0.5 * dt : dt);
+        put_hext(p, htab, tstate, (stage + 1) & 3, t + ahead);
+    }
     if (!advance) return;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -439,7 +459,9 @@ int launch_hfield_aos(mms_ctx *ctx, const float *M, const float *phi, double t, 
 
 int launch_rk4_stage(mms_ctx *ctx, int stage, const double *Mst, double *Mnext)
 {
-    MMS_CUDA_TRY(launch_k(k_rk4_stage, dim3(div_up(ctx->N, TPB)), dim3(TPB), 0, ctx->stream,
+    const bool tab = ctx->pk().n_hext > 0;
+    auto kern = !tab ? k_rk4_stage<false, false> : ctx->N <= EAGER_MAX ? k_rk4_stage<true, true> : k_rk4_stage<true, false>;
+    MMS_CUDA_TRY(launch_k(kern, dim3(div_up(ctx->N, TPB) + (tab ? 1 : 0)), dim3(TPB), 0, ctx->stream,
                           (const float *)ctx->phi, Mst, ctx->M, ctx->K, Mnext, (const uint8_t *)ctx->mat,
                           ctx->tstate, (const double *)ctx->hext, ctx->stats, ctx->gk(), ctx->pk(), stage,
                           stage == 3 ? 1 : 0));

@@ -45,6 +45,15 @@ __device__ __forceinline__ void hext_at(const PhysK &p, const double *__restrict
     H[2] = b2 * p.inv_mu0;
 }
 
+// H_ext at the time ts of an RK4 stage into the slot that the stage reads
+__device__ __forceinline__ void put_hext(const PhysK &p, const double *__restrict__ tab, double *__restrict__ tstate,
+                                         int stage, double ts)
+{
+    double he[3];
+    hext_at(p, tab, ts, he);
+    for (int c = 0; c < 3; c++) tstate[TIME_HEXT + 3 * stage + c] = he[c];
+}
+
 // half reciprocal cell sizes 1 / (2 dx), 1 / (2 dy), 1 / (2 dz): the central
 // difference weights of div_soa_cell, formed once on the host
 struct DivScale {
