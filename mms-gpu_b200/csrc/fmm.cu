@@ -131,7 +131,7 @@ struct FmmPlan {
     float *Mall = nullptr;    // [boxes of all levels][NR]
     float *Lall = nullptr;    // final locals
     float *Lpart = nullptr;   // [NSPLIT][boxes][NR] M2L partial locals
-    int4 *m2l_items = nullptr;  // {level, parity, first target, 0}: 32 targets (k_m2l_split)
+    int4 *m2l_items = nullptr;  // {level, parity, first target, 0}, class by class: 32 targets (k_m2l_split, k_m2l_res)
     int4 *res_items = nullptr;  // the same with RES_TPI targets (k_m2l_res, k_far)
     int n_res_items = 0;
     long long *lev_dev = nullptr;  // device copy of lev_off
@@ -239,6 +239,15 @@ __device__ __forceinline__ void stage_async(float *dst, const float *src, int n)
     for (int i = threadIdx.x * 4; i < n; i += blockDim.x * 4) umma::cp_async16(umma::smem_u32(dst + i), src + i, true);
     asm volatile("cp.async.commit_group;\n" ::: "memory");
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+}
+
+// a += t m, per component
+__device__ __forceinline__ void fma2(float2 &a, const float2 t, float m)
+{
+    asm("{\n.reg .b64 x, y, z;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %4};\nmov.b64 z, {%0, %1};\n"
+        "fma.rn.f32x2 z, x, y, z;\nmov.b64 {%0, %1}, z;\n}\n"
+        : "+f"(a.x), "+f"(a.y)
+        : "f"(t.x), "f"(t.y), "f"(m));
 }
 
 // One P2M output: sum over the leaf's C cells of W[c][k] q[c], w = &W[0][k]
@@ -549,143 +558,229 @@ __global__ void __launch_bounds__(32 * M2L_WARPS) k_m2l_split(const float *__res
 constexpr int RES_WARPS = 8;
 constexpr int RES_TPI = 16;  // targets per resident-M2L item
 
-// one M2L item (32 targets of one level and parity class, all 27 offsets) on
-// RES_WARPS warps; Ts = all 49 operator slots in shared memory; red =
-// RES_WARPS * 32 * (NR + 1) floats of shared scratch (may alias Ts: it is
-// written only after the last operator read)
-// one M2L item (RES_TPI = 16 targets of one level and parity class, all 27
-// offsets) on RES_WARPS warps; lane = (half, target): the 16 slots (warp,
-// half) take the class's offsets s, s + 16 (class order), the two halves of a
-// warp are added with one shuffle and the warps in a fixed order.  Ts = all
-// 49 operator slots in shared memory; red = RES_WARPS * RES_TPI * (NR + 1)
-// floats of shared scratch (may alias Ts: it is written only after the last
-// operator read)
-template <int NR_, int NE_, bool NC>
-__device__ __forceinline__ void m2l_res_item(const float *__restrict__ Mall, float *__restrict__ Lout, const float *Ts,
-                                             float *red, const int4 it, const long long *__restrict__ lev_off)
+// acc += T^T m over one n x n parity block (j-major, n even): 16-byte broadcast
+// reads and packed FMAs (two separate FP32 FMAs each), so that neither the
+// shared-memory reads nor the issue slots outweigh the other
+template <int n>
+__device__ __forceinline__ void m2l_block(const float *T, const float *m, float2 *acc)
+{
+    const float4 *row = reinterpret_cast<const float4 *>(T);
+#pragma unroll
+    for (int v = 0; v < n * n / 4; v++) {
+        const float4 t = row[v];
+        fma2(acc[4 * v % n / 2], make_float2(t.x, t.y), m[4 * v / n]);
+        fma2(acc[(4 * v + 2) % n / 2], make_float2(t.z, t.w), m[(4 * v + 2) / n]);
+    }
+}
+
+// offset i (0 .. 26) of the interaction list of parity class (px, py): rows oy =
+// py - 3 .. py + 2, in each ox = px - 3 .. px + 2 but the near ones (|ox|, |oy| < 2)
+__device__ __forceinline__ void class_offset(int px, int py, int i, int &ox, int &oy)
+{
+    // rows of 6, three of them (oy = -1, 0, 1) of 3
+    const int full = py == 0 ? 12 : 6;  // offsets before the short rows
+    int row, j;
+    bool near = false;
+    if (i < full) {
+        row = i / 6;
+        j = i % 6;
+    } else if (i < full + 9) {
+        row = full / 6 + (i - full) / 3;
+        j = (i - full) % 3;
+        near = true;
+    } else {
+        row = full / 6 + 3 + (i - full - 9) / 6;
+        j = (i - full - 9) % 6;
+    }
+    oy = py - 3 + row;
+    if (near)
+        ox = px == 0 ? (j < 2 ? j - 3 : 2) : (j < 1 ? -2 : j + 1);
+    else
+        ox = px - 3 + j;
+}
+
+// The sources of an item (TPI targets of one level and parity class: TPI
+// consecutive ones of a row, or whole rows where the level has fewer): every
+// target's 6 x 6 boxes from (2 i - 2, 2 j - 2) on, the region's boxes at pitch NR
+struct ResRegion {
+    int lev, n, nh, x0, y0, w, h;
+};
+// boxes of the largest region: one row of targets
+__host__ __device__ constexpr int res_boxes(int TPI) { return (2 * TPI + 4) * 6; }
+template <int TPI>
+__device__ __forceinline__ ResRegion res_region(const int4 it)
+{
+    ResRegion r;
+    r.lev = it.x;
+    r.n = 1 << it.x;
+    r.nh = r.n >> 1;
+    const int tw = min(r.nh, TPI), th = min(r.nh, TPI / tw);
+    r.x0 = 2 * (it.z & (r.nh - 1)) - 2;
+    r.y0 = 2 * (it.z >> (it.x - 1)) - 2;
+    r.w = 2 * tw + 4;
+    r.h = 2 * th + 4;
+    return r;
+}
+
+// the region into shared memory, zeros beyond the grid; pairs of boxes (x0 and
+// n are even, and so is every level's first box) are 16-byte chunks.  ASYNC:
+// cp.async (the caller commits and waits), else loads and stores (expansions
+// written earlier in the same kernel)
+template <int NR_, int TPI, bool ASYNC>
+__device__ __forceinline__ void m2l_res_load(const float *__restrict__ Mall, float *src, const int4 it,
+                                             const long long *__restrict__ lev_off)
+{
+    const ResRegion r = res_region<TPI>(it);
+    const float *M = Mall + lev_off[r.lev] * NR_;
+    const int per_row = r.w / 2 * (NR_ / 2);
+    for (int e = threadIdx.x; e < r.h * per_row; e += 32 * RES_WARPS) {
+        const int row = e / per_row, c = e - row * per_row, x = r.x0 + 2 * (c / (NR_ / 2)), y = r.y0 + row;
+        const bool ok = x >= 0 && x < r.n && y >= 0 && y < r.n;
+        const float *g = M + (ok ? ((long long)y * r.n + r.x0) * NR_ + 4 * c : 0);
+        float *d = src + 4 * e;
+        if (ASYNC)
+            umma::cp_async16(umma::smem_u32(d), ok ? g : Mall, ok);
+        else
+            *reinterpret_cast<float4 *>(d) = ok ? *reinterpret_cast<const float4 *>(g) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+}
+
+// one M2L item (TPI = 16 or 32 targets of one level and parity class, all 27
+// offsets) on RES_WARPS warps.  The 27 offsets go to 16 slots (i and i + 16 of
+// the class's order), slots 2 w and 2 w + 1 to warp w: to its halves (lane =
+// (half, target)), or one after the other with a lane a target; their sums are
+// added, then the warps' in a fixed order, so both forms give the same bits.
+// Ts = operators in shared memory (CLS: the class's 27, else all 49), src = the
+// item's sources (m2l_res_load).  The warps' partials (RES_WARPS TPI (NR + 1)
+// floats) take the sources' place.
+template <int NR_, int NE_, int TPI, bool CLS>
+__device__ __forceinline__ void m2l_res_item(float *__restrict__ Lout, const float *Ts, float *src, const int4 it,
+                                             const long long *__restrict__ lev_off)
 {
     constexpr int NO_ = NR_ - NE_;
     constexpr int OSZ = NE_ * NE_ + NO_ * NO_;
     constexpr int NSLOT = 2 * RES_WARPS;
-    const int lev = it.x, px = it.y & 1, py = it.y >> 1;
+    static_assert(RES_WARPS * TPI * (NR_ + 1) <= res_boxes(TPI) * NR_, "partials fit in the sources' place");
+    const ResRegion rg = res_region<TPI>(it);
+    const int px = it.y & 1, py = it.y >> 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int half = lane >> 4, tl = lane & 15, slot = 2 * warp + half;
-    const int n = 1 << lev, nh = n >> 1;
-    const long long off = lev_off[lev];
+    const int tl = lane % TPI;
+    const int n = rg.n, nh = rg.nh;
     const int ti = it.z + tl;
     const bool tvalid = ti < nh * nh;
-    const int tx = 2 * (ti % nh) + px, ty = 2 * (ti / nh) + py;
-    // this slot's offsets (s, s + 16) of the class's 27, in class order
-    int ox_l[2], oy_l[2], no = 0;
-    {
-        int idx = 0;
-        for (int oy = py - 3; oy <= py + 2; oy++)
-            for (int ox = px - 3; ox <= px + 2; ox++) {
-                if (max(abs(ox), abs(oy)) < 2) continue;
-                if ((idx++ % NSLOT) == slot && no < 2) {
-                    ox_l[no] = ox;
-                    oy_l[no] = oy;
-                    no++;
-                }
+    const int tx = 2 * (ti & (nh - 1)) + px, ty = 2 * (ti >> (rg.lev - 1)) + py;
+    auto run = [&](int slot, float2 *acc) {
+#pragma unroll
+        for (int k = 0; k < NR_ / 2; k++) acc[k] = make_float2(0.f, 0.f);
+#pragma unroll 1
+        for (int i = slot; i < 27; i += NSLOT) {
+            int ox, oy;
+            class_offset(px, py, i, ox, oy);
+            const int sb = tvalid ? (ty - oy - rg.y0) * rg.w + tx - ox - rg.x0 : 0;
+            const float2 *ms = reinterpret_cast<const float2 *>(src + sb * NR_);
+            float m[NR_];
+#pragma unroll
+            for (int v = 0; v < NR_ / 2; v++) {
+                const float2 u = ms[v];
+                m[2 * v] = u.x;
+                m[2 * v + 1] = u.y;
             }
-    }
-    float acc[NR_];
-#pragma unroll
-    for (int k = 0; k < NR_; k++) acc[k] = 0.f;
-    float m[NR_], mn[NR_];
-    auto fetch = [&](int q, float *dst) {
-        const int sx = tx - ox_l[q], sy = ty - oy_l[q];
-        const bool ok = tvalid && sx >= 0 && sy >= 0 && sx < n && sy < n;
-        const float2 *ms = reinterpret_cast<const float2 *>(Mall + (off + (long long)(ok ? sy : 0) * n + (ok ? sx : 0)) * NR_);
-#pragma unroll
-        for (int v = 0; v < NR_ / 2; v++) {
-            const float2 u = ok ? (NC ? __ldg(&ms[v]) : ms[v]) : make_float2(0.f, 0.f);
-            dst[2 * v] = u.x;
-            dst[2 * v + 1] = u.y;
+            const float *T = Ts + (CLS ? i : (oy + 3) * 7 + ox + 3) * OSZ;
+            m2l_block<NE_>(T, m, acc);
+            m2l_block<NO_>(T + NE_ * NE_, m + NE_, acc + NE_ / 2);
         }
     };
-    if (no > 0) fetch(0, m);
-    __syncthreads();
-#pragma unroll 1
-    for (int q = 0; q < 2; q++) {
-        if (q >= no) break;
-        if (q + 1 < no) fetch(q + 1, mn);
-        const float *T = Ts + ((oy_l[q] + 3) * 7 + (ox_l[q] + 3)) * OSZ;
+    float2 acc[NR_ / 2];
+    if constexpr (TPI == 16) {
+        run(2 * warp + (lane >> 4), acc);
 #pragma unroll
-        for (int j = 0; j < NE_; j++) {
-            const float2 *row = reinterpret_cast<const float2 *>(T + j * NE_);
-#pragma unroll
-            for (int v = 0; v < NE_ / 2; v++) {
-                const float2 t = row[v];
-                acc[2 * v] = fmaf(t.x, m[j], acc[2 * v]);
-                acc[2 * v + 1] = fmaf(t.y, m[j], acc[2 * v + 1]);
-            }
+        for (int k = 0; k < NR_ / 2; k++) {
+            acc[k].x += __shfl_down_sync(0xffffffffu, acc[k].x, 16);
+            acc[k].y += __shfl_down_sync(0xffffffffu, acc[k].y, 16);
         }
-        T += NE_ * NE_;
+    } else {
+        float2 up[NR_ / 2];
+        run(2 * warp, acc);
+        run(2 * warp + 1, up);
 #pragma unroll
-        for (int j = 0; j < NO_; j++) {
-            const float2 *row = reinterpret_cast<const float2 *>(T + j * NO_);
-#pragma unroll
-            for (int v = 0; v < NO_ / 2; v++) {
-                const float2 t = row[v];
-                acc[NE_ + 2 * v] = fmaf(t.x, m[NE_ + j], acc[NE_ + 2 * v]);
-                acc[NE_ + 2 * v + 1] = fmaf(t.y, m[NE_ + j], acc[NE_ + 2 * v + 1]);
-            }
+        for (int k = 0; k < NR_ / 2; k++) {
+            acc[k].x += up[k].x;
+            acc[k].y += up[k].y;
         }
-#pragma unroll
-        for (int k = 0; k < NR_; k++) m[k] = mn[k];
     }
-    // the two halves of the warp hold the same targets: lower + upper
+    float *red = src;
+    __syncthreads();  // the sources are no longer needed
+    if (lane < TPI) {
+        float *rw = red + (warp * TPI + tl) * (NR_ + 1);
 #pragma unroll
-    for (int k = 0; k < NR_; k++) acc[k] += __shfl_down_sync(0xffffffffu, acc[k], 16);
-    __syncthreads();  // (when red aliases Ts) operators no longer needed
-    if (half == 0) {
-        float *rw = red + (warp * RES_TPI + tl) * (NR_ + 1);
-#pragma unroll
-        for (int k = 0; k < NR_; k++) rw[k] = acc[k];
+        for (int k = 0; k < NR_ / 2; k++) {
+            rw[2 * k] = acc[k].x;
+            rw[2 * k + 1] = acc[k].y;
+        }
     }
     __syncthreads();
     // fixed-order sum over the warps: thread t handles (target, k) pairs
-    for (int e = threadIdx.x; e < RES_TPI * NR_; e += blockDim.x) {
-        const int t = e / NR_, k = e % NR_;
-        const int tj = it.z + t;
+    const long long off = lev_off[rg.lev];
+    for (int e = threadIdx.x; e < TPI * NR_; e += 32 * RES_WARPS) {
+        const int i = e / NR_, k = e % NR_;
+        const int tj = it.z + i;
         if (tj >= nh * nh) continue;
         float v = 0.f;
 #pragma unroll
-        for (int w = 0; w < RES_WARPS; w++) v += red[(w * RES_TPI + t) * (NR_ + 1) + k];
-        const int ux = 2 * (tj % nh) + px, uy = 2 * (tj / nh) + py;
+        for (int w = 0; w < RES_WARPS; w++) v += red[(w * TPI + i) * (NR_ + 1) + k];
+        const int ux = 2 * (tj & (nh - 1)) + px, uy = 2 * (tj >> (rg.lev - 1)) + py;
         Lout[(off + (long long)uy * n + ux) * NR_ + k] = v;
     }
     __syncthreads();
 }
 
+// CTA c takes items c / 4, .. of parity class c % 4 (nper items a class, class by
+// class in items) and keeps the class's 27 operators for all of them (one item a
+// CTA where the levels' tables differ).
 // Registers: at most 112 for NR <= 30 (P <= 4, no spills), so that one CTA
 // fits beside two k_p2p CTAs of 288 threads x 64 registers; the near field
 // runs concurrently with the M2L and, at 117 registers, the M2L's CTAs waited
-// for the near field's to finish.  256 threads per CTA.
+// for the near field's to finish.
 // lstride: floats between the operator tables of consecutive levels (tables
 // of level l at Tc + (l - 2) lstride); 0 when one table serves every level
 // (the spherical-harmonic operators, lengths in box widths).
-template <int NR_, int NE_>
+// Bound by shared-memory reads of the operators: a 16-byte broadcast feeds 4
+// FMAs a target.  Measured at 1024 x 1024 x 3, leaf 8, P = 4: sources read from
+// global memory box by box and a table of all 49 operators for each item 50 us;
+// sources staged in whole lines 46; the class's 27 operators kept, a lane a
+// target (32-target items) 37.
+template <int NR_, int NE_, int TPI>
 __global__ void __maxnreg__(NR_ <= 30 ? 112 : 255) k_m2l_res(const float *__restrict__ Mall, float *__restrict__ Lout,
                                                             const float *__restrict__ Tc, const int4 *__restrict__ items,
-                                                            const long long *__restrict__ lev_off, FmmDev f,
-                                                            long long lstride)
+                                                            const long long *__restrict__ lev_off, long long lstride,
+                                                            int nper)
 {
     constexpr int NO_ = NR_ - NE_;
     constexpr int OSZ = NE_ * NE_ + NO_ * NO_;
     extern __shared__ __align__(16) float sr[];
-    Tc += (long long)(items[blockIdx.x].x - 2) * lstride;
-    // stage the operator table with asynchronous copies: every 16-byte chunk
+    float *src = sr + 27 * OSZ;
+    const int cls = blockIdx.x & 3, step = gridDim.x >> 2;
+    int i = blockIdx.x >> 2;
+    items += cls * nper;
+    Tc += (long long)(items[i].x - 2) * lstride;
+    // stage the class's operators with asynchronous copies: every 16-byte chunk
     // in flight at once instead of one load-store round trip per chunk; the
     // table is constant, so it streams in while the predecessor finishes
-    for (int i = threadIdx.x * 4; i < 49 * OSZ; i += blockDim.x * 4)
-        umma::cp_async16(umma::smem_u32(&sr[i]), &Tc[i], true);
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    for (int q = threadIdx.x >> 5; q < 27; q += RES_WARPS) {
+        int ox, oy;
+        class_offset(cls & 1, cls >> 1, q, ox, oy);
+        const float *T = Tc + ((oy + 3) * 7 + ox + 3) * OSZ;
+        for (int e = (threadIdx.x & 31) * 4; e < OSZ; e += 128)
+            umma::cp_async16(umma::smem_u32(&sr[q * OSZ + e]), T + e, true);
+    }
     pdl_begin();
-    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    (void)f;
-    m2l_res_item<NR_, NE_, true>(Mall, Lout, sr, sr, items[blockIdx.x], lev_off);
+    for (; i < nper; i += step) {
+        m2l_res_load<NR_, TPI, true>(Mall, src, items[i], lev_off);
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();
+        m2l_res_item<NR_, NE_, TPI, true>(Lout, sr, src, items[i], lev_off);
+    }
 }
 
 // one parent box of the downward pass with a group of 4 KT threads: child
@@ -1047,7 +1142,7 @@ constexpr int far_scratch(int C)
 {
     constexpr int KT = far_kt<NR_>();
     constexpr int G = (32 * RES_WARPS) / (4 * KT);
-    const int a = C * BB, b = RES_WARPS * RES_TPI * (NR_ + 1), c = G * (4 * NR_ + 4 * KT + NR_);
+    const int a = C * BB, b = res_boxes(RES_TPI) * NR_, c = G * (4 * NR_ + 4 * KT + NR_);
     return a > b ? (a > c ? a : c) : (b > c ? b : c);
 }
 
@@ -1102,7 +1197,11 @@ __global__ void __launch_bounds__(32 * RES_WARPS) k_far(const float *__restrict_
     // M2L, every level
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
-    for (int it = blockIdx.x; it < nitems; it += gridDim.x) m2l_res_item<NR_, NE_, false>(Mall, Lpart, Tl, scr, items[it], lev_off);
+    for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
+        m2l_res_load<NR_, RES_TPI, false>(Mall, scr, items[it], lev_off);
+        __syncthreads();
+        m2l_res_item<NR_, NE_, RES_TPI, false>(Lpart, Tl, scr, items[it], lev_off);
+    }
     // L2L: level 2 from its partials, then 3 .. lend
     if (lend >= 2) {
         grid_barrier(sy);
@@ -1478,6 +1577,107 @@ __global__ void __launch_bounds__(512) k_l2p(const float *__restrict__ near, con
 #pragma unroll
     for (int i = 0; i < S; i++)
         if ((bx0 + b) * S + i < f.X) phi[row + i] = acc[i];
+}
+
+// k_l2p for grids of many leaf boxes: a CTA takes R rows of 32 / S boxes
+// (whole parents, so each parent's locals are formed once), a warp one 32-cell
+// strip of one layer, a lane one x with its R S cells along y.  Near field and
+// phi then move in whole lines, a value of V serves R boxes, and a coefficient
+// is one broadcast read.  The parents' locals are k_l2p's pmode 2; the levels
+// above come from L2L passes.  k_l2p is made for the shortest chain and bound by
+// its ancestors' serial sums and by partial lines here: 1024 x 1024 x 3, leaf 8,
+// P = 4: 115 us, this 34 us and 9 us of L2L passes.
+template <int S, int R>
+__global__ void __launch_bounds__(512) k_l2p_wide(const float *__restrict__ near, const float *__restrict__ Lpart_leaf,
+                                                  const float *__restrict__ Tl2l, const float *__restrict__ Vt,
+                                                  float *__restrict__ phi, FmmDev f, long long part_stride, int nsplit,
+                                                  const float *__restrict__ Lgp, const float *__restrict__ Lpp,
+                                                  int nnear, long long near_stride)
+{
+    extern __shared__ __align__(16) float sl[];
+    constexpr int BX = 32 / S, NB = BX * R, PX = BX / 2, NP = PX * (R / 2), GX = PX / 2, LP = NB + 1;
+    const int NE = f.NE, NO = f.NR - f.NE, NR = f.NR, np = f.nb >> 1, ng = np >> 1;
+    float *Ts = sl;                       // L2L operator blocks
+    float *Lb = Ts + 4 * (NE * NE + NO * NO);  // [NR][LP] leaf locals
+    float *Lp = Lb + NR * LP;             // [NP][NR] parent locals
+    float *Lg = Lp + NP * NR;             // [GX][NR] grandparent locals
+    const int by0 = blockIdx.y * R, bx0 = blockIdx.x * BX;
+    for (int i = threadIdx.x * 4; i < 4 * (NE * NE + NO * NO); i += blockDim.x * 4)
+        umma::cp_async16(umma::smem_u32(Ts + i), Tl2l + i, true);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    pdl_begin();
+    for (int i = threadIdx.x; i < GX * NR; i += blockDim.x) {
+        const int gc = (bx0 >> 2) + i / NR;
+        Lg[i] = gc < ng ? Lgp[((long long)(by0 >> 2) * ng + gc) * NR + i % NR] : 0.f;
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int x = bx0 * S + lane;
+    const long long cell0 = ((long long)warp * f.Y + by0 * S) * f.X + x;
+    const int rows = x < f.X ? min(R * S, f.Y - by0 * S) : 0;  // rows of the grid in this lane's column
+    float acc[R * S];
+#pragma unroll
+    for (int y = 0; y < R * S; y++) acc[y] = y < rows ? near[cell0 + (long long)y * f.X] : 0.f;
+    for (int q = 1; q < nnear; q++) {
+        const float *nq = near + q * near_stride + cell0;
+#pragma unroll
+        for (int y = 0; y < R * S; y++)
+            if (y < rows) acc[y] += nq[(long long)y * f.X];
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+    for (int i = threadIdx.x; i < NP * NR; i += blockDim.x) {
+        const int p = i / NR, k = i - p * NR, px = (bx0 >> 1) + p % PX, py = (by0 >> 1) + p / PX;
+        float v = 0.f;
+        if (px < np && py < np) {
+            const long long box = (long long)py * np + px;
+            const float first = Lpp[box * NR + k];
+            const int c = (px & 1) | ((py & 1) << 1);
+            const int blk = k >= NE, NBK = blk ? NO : NE, kk = blk ? k - NE : k;
+            const float *T = Ts + blk_base(c, NE, NO, blk);
+            const float *lg = Lg + (p % PX >> 1) * NR + (blk ? NE : 0);
+#pragma unroll 8
+            for (int j = 0; j < NBK; j++) v = fmaf(T[j * NBK + kk], lg[j], v);
+            v += first;
+            for (int q = 1; q < nsplit; q++) v += Lpp[q * part_stride + box * NR + k];
+        }
+        Lp[i] = v;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < NB * NR; i += blockDim.x) {
+        const int b = i / NR, k = i - b * NR, bx = bx0 + b % BX, by = by0 + b / BX;
+        float v = 0.f;
+        if (bx < f.nb && by < f.nb) {
+            const long long box = (long long)by * f.nb + bx;
+            const float first = Lpart_leaf[box * NR + k];
+            const int c = (bx & 1) | ((by & 1) << 1);
+            const int blk = k >= NE, NBK = blk ? NO : NE, kk = blk ? k - NE : k;
+            const float *T = Ts + blk_base(c, NE, NO, blk);
+            const float *lp = Lp + ((b / BX >> 1) * PX + (b % BX >> 1)) * NR + (blk ? NE : 0);
+#pragma unroll 8
+            for (int j = 0; j < NBK; j++) v = fmaf(T[j * NBK + kk], lp[j], v);
+            v += first;
+            for (int q = 1; q < nsplit; q++) v += Lpart_leaf[q * part_stride + box * NR + k];
+        }
+        Lb[k * LP + b] = v;
+    }
+    __syncthreads();
+    const float *lb = Lb + lane / S;
+    const float *vc = Vt + warp * S * S + lane % S;
+#pragma unroll 2
+    for (int k = 0; k < NR; k++) {
+        float l[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) l[r] = lb[k * LP + r * BX];
+#pragma unroll
+        for (int y = 0; y < S; y++) {
+            const float v = __ldg(vc + (long long)k * f.C + y * S);
+#pragma unroll
+            for (int r = 0; r < R; r++) acc[r * S + y] = fmaf(v, l[r], acc[r * S + y]);
+        }
+    }
+#pragma unroll
+    for (int y = 0; y < R * S; y++)
+        if (y < rows) phi[cell0 + (long long)y * f.X] = acc[y];
 }
 
 // ---- tensor-core M2L ------------------------------------------------------
@@ -1984,31 +2184,49 @@ int m2l_res_supported(int NR, int NE)
     return 0;
 }
 
-size_t m2l_res_smem(int NR, int NE)
+size_t m2l_res_smem(int NR, int NE, int TPI)
 {
     const int NO = NR - NE;
-    return std::max((size_t)49 * (NE * NE + NO * NO), (size_t)RES_WARPS * RES_TPI * (NR + 1)) * sizeof(float);
+    return ((size_t)27 * (NE * NE + NO * NO) + (size_t)res_boxes(TPI) * NR) * sizeof(float);
 }
 
 int m2l_res_prepare(int NR, int NE)
 {
-    const int b = (int)m2l_res_smem(NR, NE);
     cudaError_t e = cudaSuccess;
-#define X(a, c) if (NR == a && NE == c) e = cudaFuncSetAttribute(k_m2l_res<a, c>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+#define X(a, c)                                                                                    \
+    if (NR == a && NE == c) {                                                                      \
+        e = cudaFuncSetAttribute(k_m2l_res<a, c, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                 (int)m2l_res_smem(NR, NE, 16));                                   \
+        if (e == cudaSuccess)                                                                      \
+            e = cudaFuncSetAttribute(k_m2l_res<a, c, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                     (int)m2l_res_smem(NR, NE, 32));                               \
+    }
     MMS_M2L_RES_CASES(X)
 #undef X
     if (e != cudaSuccess) {
-        mms_set_error("M2L shared memory (%d B): %s", b, cudaGetErrorString(e));
+        mms_set_error("M2L shared memory: %s", cudaGetErrorString(e));
         return MMS_ERR_ARG;
     }
     return MMS_OK;
 }
 
-int m2l_res_launch(const FmmDev &f, int nitems, const float *Mall, float *Lout, const float *Tc, const int4 *items,
-                   const long long *lev, cudaStream_t st, long long lstride = 0)
+// nitems / items: 16-target items; wide: 32-target ones (one table for all
+// levels), taken where they alone fill the chip (512 x 512 x 3, leaf 4: 120 us
+// a potential with 16, 116 with 32; below, fewer items than CTAs)
+int m2l_res_launch(const FmmDev &f, int nitems, const int4 *items, int nwide, const int4 *wide, const float *Mall,
+                   float *Lout, const float *Tc, const long long *lev, cudaStream_t st, long long lstride = 0)
 {
-    const size_t sm = m2l_res_smem(f.NR, f.NE);
-#define X(a, c) if (f.NR == a && f.NE == c) { MMS_CUDA_TRY(launch_k(k_m2l_res<a, c>, dim3(nitems), dim3(32 * RES_WARPS), sm, st, Mall, Lout, Tc, items, lev, f, lstride)); return MMS_OK; }
+    const int most = f.NR <= 30 ? 2 * 148 : 148;  // CTAs the chip holds
+    const bool w = lstride == 0 && nwide >= most;
+    if (w) nitems = nwide;
+    const int ncta = lstride == 0 ? std::min(nitems, most) : nitems;
+    const size_t sm = m2l_res_smem(f.NR, f.NE, w ? 32 : 16);
+#define X(a, c)                                                                                                 \
+    if (f.NR == a && f.NE == c) {                                                                               \
+        MMS_CUDA_TRY(launch_k(w ? k_m2l_res<a, c, 32> : k_m2l_res<a, c, 16>, dim3(ncta), dim3(32 * RES_WARPS), sm, \
+                              st, Mall, Lout, Tc, w ? wide : items, lev, lstride, nitems / 4));                 \
+        return MMS_OK;                                                                                          \
+    }
     MMS_M2L_RES_CASES(X)
 #undef X
     mms_set_error("no resident M2L kernel for NR=%d", f.NR);
@@ -2028,7 +2246,7 @@ int fmm_set_carveout()
                        (const void *)k_top_m2m,    (const void *)k_top_l2l,     (const void *)k_l2l_c,
                        (const void *)k_m2l_split,  (const void *)k_m2l_gather,  (const void *)k_m2l_gemm};
     for (const void *fn : k) MMS_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, c));
-#define X(a, b) MMS_CUDA_TRY(cudaFuncSetAttribute(k_m2l_res<a, b>, cudaFuncAttributePreferredSharedMemoryCarveout, c));
+#define X(a, b) MMS_CUDA_TRY(cudaFuncSetAttribute(k_m2l_res<a, b, 16>, cudaFuncAttributePreferredSharedMemoryCarveout, c)); MMS_CUDA_TRY(cudaFuncSetAttribute(k_m2l_res<a, b, 32>, cudaFuncAttributePreferredSharedMemoryCarveout, c));
     MMS_M2L_RES_CASES(X)
 #undef X
 #define X(S_, B_)                                                                                            \
@@ -2220,7 +2438,7 @@ int fmm_plan_create(mms_ctx *ctx)
     }
     // levels, work items
     pl->lev_off.assign(f.L + 2, 0);
-    long long tot = 0;
+    long long tot = 1;  // so that levels 2 .. start on an even box: 16-byte aligned expansions of any (even) NR
     for (int l = 0; l <= f.L; l++) {
         pl->lev_off[l] = tot;
         tot += (long long)(1 << l) * (1 << l);
@@ -2228,18 +2446,18 @@ int fmm_plan_create(mms_ctx *ctx)
     pl->lev_off[f.L + 1] = tot;
     pl->nbox_total = tot;
     std::vector<int4> items;
-    for (int l = 2; l <= f.L; l++) {
-        const int nh = (1 << l) / 2;
-        for (int par = 0; par < 4; par++)
+    for (int par = 0; par < 4; par++)
+        for (int l = 2; l <= f.L; l++) {
+            const int nh = (1 << l) / 2;
             for (int t0 = 0; t0 < nh * nh; t0 += 32) items.push_back(make_int4(l, par, t0, 0));
-    }
+        }
     pl->n_m2l_items = (int)items.size();
     std::vector<int4> ritems;
-    for (int l = 2; l <= f.L; l++) {
-        const int nh = (1 << l) / 2;
-        for (int par = 0; par < 4; par++)
+    for (int par = 0; par < 4; par++)
+        for (int l = 2; l <= f.L; l++) {
+            const int nh = (1 << l) / 2;
             for (int t0 = 0; t0 < nh * nh; t0 += RES_TPI) ritems.push_back(make_int4(l, par, t0, 0));
-    }
+        }
     pl->n_res_items = (int)ritems.size();
 
     // tensor-core M2L rows: every box of levels >= 2, grouped by parity class
@@ -2549,7 +2767,35 @@ static int p2m_up(const FmmPlan *pl) { return l2p_up(pl) && pl->d.NR <= 32; }
 static int top_two(const FmmPlan *pl) { return pl->d.NR <= 32 && !pl->far_fused; }
 // L2P also forms levels 2 .. L-2 of each CTA's ancestors (pmode 4): no L2L
 // launch at all between the M2L and L2P
-static int l2p_top(const FmmPlan *pl) { return l2p_up(pl) && pl->d.L >= 4; }
+
+// k_l2p_wide and the L2L passes it needs, from the grid on where its CTAs of
+// 32 x 16 columns fill the chip.  A potential of P = 4 and 3 layers, k_l2p with
+// the levels it forms by itself against this: 256 x 256 (leaf 8) 30 us against
+// 34, 320 x 320 50 against 55, 352 x 352 61 against 56, 1024 x 1024 282 against
+// 206; at leaf 4 52 against 54, 95 against 97, 545 against 412
+static int l2p_wide(const FmmPlan *pl)
+{
+    const FmmDev &f = pl->d;
+    return l2p_up(pl) && f.L >= 4 && (f.s == 4 || f.s == 8) && f.Z <= 16 &&
+           (long long)div_up(f.X, 32) * div_up(f.Y, 16) >= 240;
+}
+static int l2p_top(const FmmPlan *pl) { return l2p_up(pl) && pl->d.L >= 4 && !l2p_wide(pl); }
+
+template <int S, int R>
+static int l2p_wide_launch(const FmmPlan *pl, const float *near, const float *Lgp, const float *Lpp, float *phi,
+                           int nsplit, int nnear, long long near_stride, cudaStream_t st)
+{
+    const FmmDev &f = pl->d;
+    constexpr int BX = 32 / S, NB = BX * R, NP = NB / 4, GX = BX / 4;
+    const size_t smem = (4 * ((size_t)f.NE * f.NE + (size_t)(f.NR - f.NE) * (f.NR - f.NE)) +
+                         (size_t)f.NR * (NB + 1 + NP + GX)) * sizeof(float);
+    MMS_CUDA_TRY(cudaFuncSetAttribute(k_l2p_wide<S, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    MMS_CUDA_TRY(launch_k(k_l2p_wide<S, R>, dim3(div_up(f.X, 32), div_up(f.Y, R * S)),
+                          dim3(32 * f.Z), smem, st, near, (const float *)(pl->Lpart + pl->lev_off[f.L] * f.NR),
+                          (const float *)pl->Tl2l, (const float *)pl->Vt, phi, f, pl->nbox_total * f.NR, nsplit, Lgp, Lpp,
+                          nnear, near_stride));
+    return MMS_OK;
+}
 
 // L2P of the far field onto the near field already in pl->near
 static int l2p_launch_far(mms_ctx *ctx, const float *rho, float *phi)
@@ -2565,6 +2811,12 @@ static int l2p_launch_far(mms_ctx *ctx, const float *rho, float *phi)
     const float *Lgp = f.L >= 4 ? pl->Lall + pl->lev_off[f.L - 2] * f.NR : nullptr;
     const float *Lpp = f.L > 2 ? pl->Lpart + pl->lev_off[f.L - 1] * f.NR : nullptr;
     const float *near = pl->p2p_tc ? pl->near3 : pl->near;
+    if (l2p_wide(pl)) {
+        MMS_TRY((f.s == 8 ? l2p_wide_launch<8, 2> : l2p_wide_launch<4, 4>)(pl, near, Lgp, Lpp, phi, nsplit,
+                                                                          pl->p2p_tc ? 3 : 1, ctx->N, ctx->stream));
+        MMS_LAUNCH_CHECK(ctx);
+        return MMS_OK;
+    }
     MMS_TRY(l2p_launch(f, nbx, nby, near, pl->Lpart + pl->lev_off[f.L] * f.NR, Lpar, pl->Tl2l, pl->Vt, phi,
                        pl->nbox_total * f.NR, nsplit, pmode, Lgp, Lpp, pl->p2p_tc ? 3 : 1, ctx->N, pl->Lpart,
                        pl->lev_dev, ctx->stream));
@@ -2710,8 +2962,8 @@ static int launch_fmm_stage(mms_ctx *ctx, int stage, const float *rho, float *ph
             break;
         }
         if (pl->m2l_resident) {
-            MMS_TRY(m2l_res_launch(f, pl->n_res_items, pl->Mall, pl->Lpart, pl->Tm2lc, pl->res_items, pl->lev_dev,
-                                   ctx->stream));
+            MMS_TRY(m2l_res_launch(f, pl->n_res_items, pl->res_items, pl->n_m2l_items, pl->m2l_items, pl->Mall,
+                                   pl->Lpart, pl->Tm2lc, pl->lev_dev, ctx->stream));
         } else {
             const int NBmax = std::max(f.NE, f.NR - f.NE);
             const int KPmax = std::max(pl->KPb[0], pl->KPb[1]);
@@ -3231,8 +3483,8 @@ int farnet_launch(mms_ctx *ctx, const float *rho, float *phi)
     FmmDev fn = f;
     fn.NR = NR;
     fn.NE = NE;
-    MMS_TRY(m2l_res_launch(fn, pl->n_res_items, pl->fnM, pl->fnLp, pl->fnM2L, pl->res_items, pl->lev_dev, ctx->stream,
-                           49LL * OSZ));
+    MMS_TRY(m2l_res_launch(fn, pl->n_res_items, pl->res_items, pl->n_m2l_items, pl->m2l_items, pl->fnM, pl->fnLp,
+                           pl->fnM2L, pl->lev_dev, ctx->stream, 49LL * OSZ));
     MMS_LAUNCH_CHECK(ctx);
     MMS_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, pl->ev_join, 0));
     const unsigned ndown = f.L > 2 ? 1u << (2 * (f.L - 1)) : 1u << (2 * f.L);
