@@ -589,8 +589,9 @@ int mms_hfield_dev(mms_ctx *ctx, const float *M, float *H, float *charge, float 
     if (ctx->p.demag && ctx->s.kind == MMS_SOLVER_DIRECT) {
         MMS_TRY(launch_potential_direct_aos(ctx, M, charge, phi));
     } else if (ctx->p.demag) {
-        MMS_TRY(launch_divergence_aos(ctx, M, rho));
+        MMS_TRY(launch_divergence_aos(ctx, M, rho, true));
         MMS_TRY(launch_potential(ctx, rho, phi));
+        fmm_split_written(ctx, nullptr);
     }
     MMS_TRY(launch_hfield_aos(ctx, M, phi, t, H));
     if (!potential) ctx->phi_valid = false;  // ctx->phi no longer holds the state's potential
@@ -622,8 +623,9 @@ int mms_hfield_host(mms_ctx *ctx, const float *M, float *H, float *charge, float
     if (ctx->p.demag && ctx->s.kind == MMS_SOLVER_DIRECT) {
         MMS_TRY(launch_potential_direct_aos(ctx, ctx->vecA, charge ? ctx->rho : nullptr, ctx->phi));
     } else if (ctx->p.demag) {
-        MMS_TRY(launch_divergence_aos(ctx, ctx->vecA, ctx->rho));
+        MMS_TRY(launch_divergence_aos(ctx, ctx->vecA, ctx->rho, true));
         MMS_TRY(launch_potential(ctx, ctx->rho, ctx->phi));
+        fmm_split_written(ctx, nullptr);
     }
     MMS_TRY(launch_hfield_aos(ctx, ctx->vecA, ctx->phi, t, ctx->vecB));
     ctx->phi_valid = false;

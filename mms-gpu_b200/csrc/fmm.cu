@@ -241,6 +241,14 @@ __device__ __forceinline__ void stage_async(float *dst, const float *src, int n)
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 }
 
+// v + p[0] + p[stride] + ..: n partials, one after the other, their loads in flight together
+__device__ __forceinline__ float add_parts(float v, const float *__restrict__ p, long long stride, int n)
+{
+#pragma unroll 8
+    for (int q = 0; q < n; q++) v += p[q * stride];
+    return v;
+}
+
 // a += t m, per component
 __device__ __forceinline__ void fma2(float2 &a, const float2 t, float m)
 {
@@ -397,6 +405,128 @@ __global__ void __launch_bounds__(512) k_p2m_row(const float *__restrict__ rho, 
     const int pc = (bx0 >> 1) + grp;
     float *Mc = scr + grp * (4 * f.NR + 4 * KT), *red = Mc + 4 * f.NR;
     m2m_reduce(Mall, Ts, Mc, red, off_par, blockIdx.y * np + pc, f, t, KT, grp < PB / 2 && pc < np);
+}
+
+// k_p2m_row for grids of many leaf boxes: a CTA takes the 32 x 16 columns of
+// k_l2p_wide.  The charges are staged as [4 boxes of a row][cell], so that a
+// thread (4 boxes, one coefficient) has 16 sums from one weight (through L1,
+// where every CTA of the SM finds it) and one 16-byte broadcast a cell.  With
+// up the parents follow, thread per (parent, coefficient).  Per output the
+// arithmetic of p2m_dot and m2m_reduce, so the same bits.
+// Shared memory: charges [NB / 4][C][4], (up) the leaves' expansions [NB][NR],
+// (leaf side 8) the interleaved sums [4][NB / 4][NR][4].
+template <int S, int R, bool DIV>
+__global__ void __launch_bounds__(256) k_p2m_wide(const float *__restrict__ rho, const float *__restrict__ Wt,
+                                                  float *__restrict__ Mall, long long off_leaf, FmmDev f, int wsm, int up,
+                                                  const float *__restrict__ Tm2m, long long off_par, DivSrc dv)
+{
+    extern __shared__ __align__(16) float q[];
+    constexpr int BX = 32 / S, NB = BX * R, PX = BX / 2, NP = PX * (R / 2);
+    const int NR = f.NR, NE = f.NE, NO = NR - NE, C = f.C;
+    float *Mc = q + NB * C;
+    float *sw = Mc + (up ? NB * NR : 0) + (S == 8 ? 4 * NB * NR : 0);
+    // weights (wsm) and operators, constant, stream in while the predecessor finishes
+    const float *W = Wt;
+    if (wsm) {
+        for (int i = threadIdx.x * 4; i < C * NR; i += blockDim.x * 4) umma::cp_async16(umma::smem_u32(sw + i), Wt + i, true);
+        W = sw;
+        sw += C * NR;
+    }
+    if (up)
+        for (int i = threadIdx.x * 4; i < 4 * (NE * NE + NO * NO); i += blockDim.x * 4)
+            umma::cp_async16(umma::smem_u32(sw + i), Tm2m + i, true);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    pdl_begin();
+    const int bx0 = blockIdx.x * BX, by0 = blockIdx.y * R;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int x = bx0 * S + lane, b = lane / S, rows = f.Z * R * S;
+    constexpr int U = 8;  // rows a warp has in flight
+    for (int r0 = warp; r0 < rows; r0 += U * nw) {
+        float v[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int row = r0 + u * nw, z = row / (R * S), y = by0 * S + row % (R * S);
+            const bool in = row < rows && x < f.X && y < f.Y;
+            if (DIV)
+                v[u] = in ? div_value(dv, x, y, z) : 0.f;
+            else
+                v[u] = in ? rho[((long long)z * f.Y + y) * f.X + x] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int row = r0 + u * nw, z = row / (R * S), yy = row % (R * S), y = by0 * S + yy;
+            if (row >= rows) break;
+            const int box = yy / S * BX + b, cell = (z * S + yy % S) * S + lane % S;
+            q[((box >> 2) * C + cell) * 4 + (box & 3)] = v[u];
+            if (DIV && x < f.X && y < f.Y) div_store(dv, x, y, z, v[u]);
+        }
+    }
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncthreads();
+    float *Mleaf = Mall + off_leaf * NR;
+    // SPLIT (few outputs a CTA): a thread has one of the four interleaved sums
+    constexpr int SPLIT = S == 8 ? 4 : 1;
+    const int n = NB / 4 * NR;
+    float4 *part = reinterpret_cast<float4 *>(Mc + (up ? NB * NR : 0));  // [4][n], SPLIT
+    auto put = [&](int e, const float4 o4) {
+        const int g = e / NR, k = e - g * NR;
+        const float o[4] = {o4.x, o4.y, o4.z, o4.w};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int bb = 4 * g + i, bx = bx0 + bb % BX, by = by0 + bb / BX;
+            if (bx < f.nb && by < f.nb) Mleaf[((long long)by * f.nb + bx) * NR + k] = o[i];
+            if (up) Mc[bb * NR + k] = o[i];
+        }
+    };
+    auto join = [](const float4 a, const float4 b, const float4 c, const float4 d) {
+        return make_float4((a.x + b.x) + (c.x + d.x), (a.y + b.y) + (c.y + d.y), (a.z + b.z) + (c.z + d.z),
+                           (a.w + b.w) + (c.w + d.w));
+    };
+    for (int e0 = threadIdx.x; e0 < n * SPLIT; e0 += blockDim.x) {
+        const int sp = e0 / n, e = e0 - sp * n, g = e / NR, k = e - g * NR;
+        const float4 *qq = reinterpret_cast<const float4 *>(q) + g * C + sp;
+        const float *w = W + sp * NR + k;
+        float4 a[4 / SPLIT];
+#pragma unroll
+        for (int i = 0; i < 4 / SPLIT; i++) a[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll(2 * SPLIT)
+        for (int c = 0; c < C; c += 4)  // (C is a multiple of 16)
+#pragma unroll
+            for (int i = 0; i < 4 / SPLIT; i++) {
+                const float wc = w[(c + i) * NR];
+                const float4 t = qq[c + i];
+                a[i].x = fmaf(wc, t.x, a[i].x);
+                a[i].y = fmaf(wc, t.y, a[i].y);
+                a[i].z = fmaf(wc, t.z, a[i].z);
+                a[i].w = fmaf(wc, t.w, a[i].w);
+            }
+        if constexpr (SPLIT == 1)
+            put(e, join(a[0], a[1], a[2], a[3]));
+        else
+            part[e0] = a[0];
+    }
+    if (SPLIT > 1) {
+        __syncthreads();
+        for (int e = threadIdx.x; e < n; e += blockDim.x) put(e, join(part[e], part[n + e], part[2 * n + e], part[3 * n + e]));
+    }
+    if (!up) return;
+    __syncthreads();
+    const int np = f.nb >> 1;
+    for (int e = threadIdx.x; e < NP * NR; e += blockDim.x) {
+        const int p = e / NR, k = e - p * NR, px = (bx0 >> 1) + p % PX, py = (by0 >> 1) + p / PX;
+        if (px >= np || py >= np) continue;
+        const int blk = k >= NE, NBK = blk ? NO : NE, kk = blk ? k - NE : k;
+        float v[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const float *T = sw + c * (NE * NE + NO * NO) + (blk ? NE * NE : 0) + kk;
+            const float *m = Mc + ((2 * (p / PX) + (c >> 1)) * BX + 2 * (p % PX) + (c & 1)) * NR + (blk ? NE : 0);
+            v[c] = 0.f;
+#pragma unroll 8
+            for (int j = 0; j < NBK; j++) v[c] = fmaf(T[j * NBK], m[j], v[c]);
+        }
+        Mall[(off_par + (long long)py * np + px) * NR + k] = (v[0] + v[1]) + (v[2] + v[3]);
+    }
 }
 
 // M2M: CTA per parent box, thread per (child c, output coefficient k).  The
@@ -804,9 +934,7 @@ __device__ __forceinline__ void l2l_item(float *__restrict__ Lfin, const float *
         for (int j = 0; j < NB; j++) acc = fmaf(T[j * NB + kk], lp[j], acc);
         const int cx = 2 * (pb % np) + (c & 1), cy = 2 * (pb / np) + (c >> 1);
         const long long b = off_c + (long long)cy * nc + cx;
-        float v = acc;
-        for (int g = 0; g < nsplit; g++) v += Lpart[g * part_stride + b * f.NR + k];
-        Lfin[b * f.NR + k] = v;
+        Lfin[b * f.NR + k] = add_parts(acc, Lpart + b * f.NR + k, part_stride, nsplit);
     }
     __syncthreads();
 }
@@ -816,9 +944,7 @@ __device__ __forceinline__ void l2l_top_box(float *__restrict__ Lfin, const floa
                                             long long part_stride, int nsplit, const FmmDev &f, int t, int nt)
 {
     for (int k = t; k < f.NR; k += nt) {
-        float v = 0.f;
-        for (int g = 0; g < nsplit; g++) v += Lpart[g * part_stride + b * f.NR + k];
-        Lfin[b * f.NR + k] = v;
+        Lfin[b * f.NR + k] = add_parts(0.f, Lpart + b * f.NR + k, part_stride, nsplit);
     }
 }
 
@@ -1470,17 +1596,15 @@ __global__ void __launch_bounds__(512) k_l2p(const float *__restrict__ near, con
                         for (int j = 0; j < NB; j++) a2 = fmaf(T[j * NB + kk], lp[j], a2);
                         v = a2;
                     }
-                    for (int q = 0; q < nsplit; q++) {
-                        float pq;
-                        if (q == 0 && i == (int)threadIdx.x && l - 2 < NPF) {
-                            pq = apre[0];
+                    const float *pb = Lpart_all + box * f.NR + k;
+                    if (i == (int)threadIdx.x && l - 2 < NPF && nsplit > 0) {
+                        float pq = apre[0];
 #pragma unroll
-                            for (int u = 1; u < NPF; u++)
-                                if (l - 2 == u) pq = apre[u];
-                        } else {
-                            pq = Lpart_all[q * part_stride + box * f.NR + k];
-                        }
-                        v += pq;
+                        for (int u = 1; u < NPF; u++)
+                            if (l - 2 == u) pq = apre[u];
+                        v = add_parts(v + pq, pb + part_stride, part_stride, nsplit - 1);
+                    } else {
+                        v = add_parts(v, pb, part_stride, nsplit);
                     }
                 }
                 dst[i] = v;
@@ -1508,8 +1632,9 @@ __global__ void __launch_bounds__(512) k_l2p(const float *__restrict__ near, con
                     v = a2;
                 }
                 const long long pbox = (long long)prow * np + pc;
-                for (int q = 0; q < nsplit; q++)
-                    v += (q == 0 && i == (int)threadIdx.x) ? ppre : Lpp[q * part_stride + pbox * f.NR + k];
+                const float *pp = Lpp + pbox * f.NR + k;
+                v = i == (int)threadIdx.x && nsplit > 0 ? add_parts(v + ppre, pp + part_stride, part_stride, nsplit - 1)
+                                                        : add_parts(v, pp, part_stride, nsplit);
             }
             Lp[i] = v;
         }
@@ -1527,8 +1652,9 @@ __global__ void __launch_bounds__(512) k_l2p(const float *__restrict__ near, con
                 const float *lp = Lp + (bb >> 1) * f.NR + boff;
                 for (int j = 0; j < NB; j++) v = fmaf(T[j * NB + kk], lp[j], v);
             }
-            for (int q = 0; q < nsplit; q++)
-                v += (q == 0 && i == (int)threadIdx.x) ? lpre : Lpart_leaf[q * part_stride + box * f.NR + k];
+            const float *pb = Lpart_leaf + box * f.NR + k;
+            v = i == (int)threadIdx.x && nsplit > 0 ? add_parts(v + lpre, pb + part_stride, part_stride, nsplit - 1)
+                                                    : add_parts(v, pb, part_stride, nsplit);
         }
         Lb[i] = v;
     }
@@ -1637,8 +1763,7 @@ __global__ void __launch_bounds__(512) k_l2p_wide(const float *__restrict__ near
             const float *lg = Lg + (p % PX >> 1) * NR + (blk ? NE : 0);
 #pragma unroll 8
             for (int j = 0; j < NBK; j++) v = fmaf(T[j * NBK + kk], lg[j], v);
-            v += first;
-            for (int q = 1; q < nsplit; q++) v += Lpp[q * part_stride + box * NR + k];
+            v = add_parts(v + first, Lpp + part_stride + box * NR + k, part_stride, nsplit - 1);
         }
         Lp[i] = v;
     }
@@ -1655,8 +1780,7 @@ __global__ void __launch_bounds__(512) k_l2p_wide(const float *__restrict__ near
             const float *lp = Lp + ((b / BX >> 1) * PX + (b % BX >> 1)) * NR + (blk ? NE : 0);
 #pragma unroll 8
             for (int j = 0; j < NBK; j++) v = fmaf(T[j * NBK + kk], lp[j], v);
-            v += first;
-            for (int q = 1; q < nsplit; q++) v += Lpart_leaf[q * part_stride + box * NR + k];
+            v = add_parts(v + first, Lpart_leaf + part_stride + box * NR + k, part_stride, nsplit - 1);
         }
         Lb[k * LP + b] = v;
     }
@@ -1716,15 +1840,15 @@ __global__ void k_m2l_gather(const float *__restrict__ Mall, __nv_bfloat16 *__re
     // one thread per run of 8 coefficients of one offset: 16-byte stores of
     // hi, hi and lo (NBp and K are multiples of 8, rows start 16-B aligned)
     const int cpq = NBp >> 3, per_row = 27 * cpq;
-    const long long total = (long long)rows * per_row;
-    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-         e += (long long)gridDim.x * blockDim.x) {
-        const int r = (int)(e / per_row), c = (int)(e % per_row);
-        const int q = c / cpq, j0 = (c % cpq) * 8;
+    const unsigned total = (unsigned)rows * per_row;  // (one each for the grid's threads)
+    pdl_begin();
+    for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
+        const int r = (int)(e / per_row), c = (int)(e - (unsigned)r * per_row);
+        const int q = c / cpq, j0 = (c - q * cpq) * 8;
         const int4 ri = rowinfo[r];
         const int lev = ri.x, par = ri.y & 3, t = ri.z;
         const int n = 1 << lev, nh = n >> 1;
-        const int tx = 2 * (t % nh) + (par & 1), ty = 2 * (t / nh) + (par >> 1);
+        const int tx = 2 * (t & (nh - 1)) + (par & 1), ty = 2 * (t >> (lev - 1)) + (par >> 1);
         const int sx = tx - sox[par][q], sy = ty - soy[par][q];
         float v[8];
 #pragma unroll
@@ -1732,8 +1856,12 @@ __global__ void k_m2l_gather(const float *__restrict__ Mall, __nv_bfloat16 *__re
         if (sx >= 0 && sy >= 0 && sx < n && sy < n) {
             const float *src = Mall + (lev_off[lev] + (long long)sy * n + sx) * f.NR + boff + j0;
 #pragma unroll
-            for (int i = 0; i < 8; i++)
-                if (j0 + i < NB) v[i] = __ldg(src + i);
+            for (int i = 0; i < 8; i += 2)  // NB, NR and the blocks' first coefficients are even
+                if (j0 + i < NB) {
+                    const float2 u = __ldg(reinterpret_cast<const float2 *>(src + i));
+                    v[i] = u.x;
+                    v[i + 1] = u.y;
+                }
         }
         __align__(16) __nv_bfloat16 hi[8], lo[8];
 #pragma unroll
@@ -2031,6 +2159,7 @@ __global__ void __launch_bounds__(128) k_m2l_gemm(const TcGroup *__restrict__ gr
     extern __shared__ uint8_t raw[];
     const TcGroup g = groups[blockIdx.z];
     const int m0 = blockIdx.x * umma::BM;
+    pdl_begin();
     if (m0 >= g.M) return;  // before any tensor-memory allocation
     const int ktiles = (g.K + umma::BK - 1) / umma::BK, per = (ktiles + ksplit - 1) / ksplit;
     const int k0 = blockIdx.y * per * umma::BK;
@@ -2264,6 +2393,7 @@ int fmm_default_leaf(int P, int X, int Y);
 int far_prepare(mms_ctx *ctx, FmmPlan *pl);
 static int l2p_up(const FmmPlan *pl);
 static int l2p_top(const FmmPlan *pl);
+static int l2p_wide(const FmmPlan *pl);
 static int p2m_up(const FmmPlan *pl);
 
 int fmm_plan_create(mms_ctx *ctx)
@@ -2585,6 +2715,11 @@ int fmm_plan_create(mms_ctx *ctx)
         MMS_CUDA_TRY(cudaFuncSetAttribute(k_p2m_row<4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
         MMS_CUDA_TRY(cudaFuncSetAttribute(k_p2m_row<BB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
         MMS_CUDA_TRY(cudaFuncSetAttribute(k_p2m_row<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+        const void *wide[] = {(const void *)k_p2m_wide<8, 2, false>, (const void *)k_p2m_wide<8, 2, true>,
+                              (const void *)k_p2m_wide<4, 4, false>, (const void *)k_p2m_wide<4, 4, true>,
+                              (const void *)k_l2p_wide<8, 2>, (const void *)k_l2p_wide<4, 4>};
+        for (const void *k : wide)
+            MMS_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     }
     {
         const size_t tsz = 4 * cstride;
@@ -2789,7 +2924,6 @@ static int l2p_wide_launch(const FmmPlan *pl, const float *near, const float *Lg
     constexpr int BX = 32 / S, NB = BX * R, NP = NB / 4, GX = BX / 4;
     const size_t smem = (4 * ((size_t)f.NE * f.NE + (size_t)(f.NR - f.NE) * (f.NR - f.NE)) +
                          (size_t)f.NR * (NB + 1 + NP + GX)) * sizeof(float);
-    MMS_CUDA_TRY(cudaFuncSetAttribute(k_l2p_wide<S, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     MMS_CUDA_TRY(launch_k(k_l2p_wide<S, R>, dim3(div_up(f.X, 32), div_up(f.Y, R * S)),
                           dim3(32 * f.Z), smem, st, near, (const float *)(pl->Lpart + pl->lev_off[f.L] * f.NR),
                           (const float *)pl->Tl2l, (const float *)pl->Vt, phi, f, pl->nbox_total * f.NR, nsplit, Lgp, Lpp,
@@ -2878,6 +3012,20 @@ static int p2m_launch(mms_ctx *ctx, const float *rho, const DivSrc *dv)
         block(up ? (PB / 2) * 4 * KT : std::min(512, ((PB * f.NR + 31) / 32) * 32));
     const long long off_par = up ? pl->lev_off[f.L - 1] : 0LL;
     const DivSrc d0 = dv ? *dv : DivSrc{};
+    if (l2p_wide(pl)) {
+        const int NB = 32 / f.s * (16 / f.s);
+        const int wide_w = (size_t)f.C * f.NR * sizeof(float) <= 40 * 1024;
+        const size_t wide_smem = ((size_t)NB * (f.C + (up ? f.NR : 0) + (f.s == 8 ? 4 * f.NR : 0)) +
+                                  (wide_w ? (size_t)f.C * f.NR : 0) + (up ? tsz : 0)) * sizeof(float);
+        const int thr = std::min(256, (NB / 4 * f.NR * (f.s == 8 ? 4 : 1) + 31) / 32 * 32);
+        auto kern = f.s == 8 ? (dv ? k_p2m_wide<8, 2, true> : k_p2m_wide<8, 2, false>)
+                             : (dv ? k_p2m_wide<4, 4, true> : k_p2m_wide<4, 4, false>);
+        MMS_CUDA_TRY(launch_k(kern, dim3(div_up(f.X, 32), div_up(f.Y, 16)), dim3(thr), wide_smem, ctx->stream, rho,
+                              (const float *)pl->Wt, pl->Mall, leaf_off, f, wide_w, up, (const float *)pl->Tm2m, off_par,
+                              d0));
+        MMS_LAUNCH_CHECK(ctx);
+        return MMS_OK;
+    }
 #define P2M_ARGS grid, block, smem, ctx->stream, rho, (const float *)pl->Wt, pl->Mall, leaf_off, f, wsm, up, \
                  (const float *)pl->Tm2m, off_par, d0
     if (PB == 4 && dv)
@@ -2951,13 +3099,14 @@ static int launch_fmm_stage(mms_ctx *ctx, int stage, const float *rho, float *ph
     case 2: {
         if (pl->m2l_tc) {
             const long long runs = (long long)pl->tc_rows * 27 * (std::max(pl->tcNBp[0], pl->tcNBp[1]) / 8);
-            k_m2l_gather<<<dim3((unsigned)div_up(runs, 256), 2), 256, 0, ctx->stream>>>(
-                pl->Mall, pl->tcA[0], pl->tcA[1], pl->tc_rowinfo, pl->lev_dev, f, pl->tc_rows, pl->tcK[0], pl->tcK[1],
-                pl->tcNBp[0], pl->tcNBp[1]);
+            MMS_CUDA_TRY(launch_k(k_m2l_gather, dim3((unsigned)div_up(runs, 256), 2), dim3(256), 0, ctx->stream,
+                                  (const float *)pl->Mall, pl->tcA[0], pl->tcA[1], (const int4 *)pl->tc_rowinfo,
+                                  (const long long *)pl->lev_dev, f, pl->tc_rows, pl->tcK[0], pl->tcK[1],
+                                  pl->tcNBp[0], pl->tcNBp[1]));
             MMS_LAUNCH_CHECK(ctx);
-            k_m2l_gemm<<<dim3(div_up(pl->tc_maxm, umma::BM), pl->tc_ksplit, 8), 128,
-                         sizeof(umma::Smem<64, TC_STAGES>) + 1024, ctx->stream>>>(pl->tc_groups, pl->tc_ksplit,
-                                                                                 part_stride);
+            MMS_CUDA_TRY(launch_k(k_m2l_gemm, dim3(div_up(pl->tc_maxm, umma::BM), pl->tc_ksplit, 8), dim3(128),
+                                  sizeof(umma::Smem<64, TC_STAGES>) + 1024, ctx->stream,
+                                  (const TcGroup *)pl->tc_groups, pl->tc_ksplit, part_stride));
             MMS_LAUNCH_CHECK(ctx);
             break;
         }

@@ -175,7 +175,9 @@ struct mms_ctx {
 // ---------------------------------------------------------------------------
 // kernel entry points (host-side launchers); all asynchronous on ctx->stream
 int launch_divergence_soa(mms_ctx *ctx, const double *M, float *rho);
-int launch_divergence_aos(mms_ctx *ctx, const float *M, float *rho);
+// potential_next: a potential of rho follows at once; where the near field takes
+// rho's BF16 split, the divergence writes it too
+int launch_divergence_aos(mms_ctx *ctx, const float *M, float *rho, bool potential_next = false);
 int launch_gradient_aos(mms_ctx *ctx, const float *phi, double c, float *H);
 int launch_exchange_aos(mms_ctx *ctx, const float *M, float *H);
 int launch_hfield_aos(mms_ctx *ctx, const float *M, const float *phi, double t, float *H);

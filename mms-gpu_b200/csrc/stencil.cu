@@ -29,13 +29,23 @@ constexpr int TPB = 256;
 // ---- FP32 AoS, reference operation order ---------------------------------
 
 // vector_functions.cpp:8-28
-__global__ void k_div_aos(const float *__restrict__ M, float *__restrict__ rho, GridK g, float dx, float dy, float dz)
+// with rhi also the BF16 split of rho, as k_div_soa
+__global__ void __launch_bounds__(TPB) k_div_aos(const float *__restrict__ M, float *__restrict__ rho, GridK g, DivAos d,
+                                                 __nv_bfloat16 *__restrict__ rhi, __nv_bfloat16 *__restrict__ rlo,
+                                                 int nbx, int nby)
 {
     long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (i >= g.N) return;
     int x, y, z;
     cell_xyz(i, g, x, y, z);
-    rho[i] = div_aos_cell(M, i, x, y, z, g, DivAos{dx, dy, dz});
+    const float v = div_aos_cell(M, i, x, y, z, g, d);
+    rho[i] = v;
+    if (rhi) {
+        const long long j = ntc_index(x, y, z, nbx, nby);
+        const __nv_bfloat16 h = __float2bfloat16_rn(v);
+        rhi[j] = h;
+        rlo[j] = __float2bfloat16_rn(v - __bfloat162float(h));
+    }
 }
 
 // vector_functions.cpp:31-54; c is the reference's fptype constant_multiple
@@ -413,12 +423,17 @@ PhysK mms_ctx::pk() const
     return k;
 }
 
-int launch_divergence_aos(mms_ctx *ctx, const float *M, float *rho)
+int launch_divergence_aos(mms_ctx *ctx, const float *M, float *rho, bool potential_next)
 {
-    fmm_split_written(ctx, nullptr);  // rho changes without its BF16 split
-    k_div_aos<<<div_up(ctx->N, TPB), TPB, 0, ctx->stream>>>(M, rho, ctx->gk(), (float)ctx->g.dx, (float)ctx->g.dy,
-                                                           (float)ctx->g.dz);
+    void *hi = nullptr, *lo = nullptr;
+    int nbx = 0, nby = 0;
+    const int split = potential_next && fmm_split_target(ctx, &hi, &lo, &nbx, &nby);
+    k_div_aos<<<div_up(ctx->N, TPB), TPB, 0, ctx->stream>>>(
+        M, rho, ctx->gk(), DivAos{(float)ctx->g.dx, (float)ctx->g.dy, (float)ctx->g.dz},
+        (__nv_bfloat16 *)(split ? hi : nullptr), (__nv_bfloat16 *)(split ? lo : nullptr), nbx, nby);
     MMS_LAUNCH_CHECK(ctx);
+    // (without the split rho changes all the same)
+    fmm_split_written(ctx, split ? rho : nullptr);
     return MMS_OK;
 }
 
