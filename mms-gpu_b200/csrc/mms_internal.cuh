@@ -141,6 +141,7 @@ struct mms_ctx {
     double *stats = nullptr;                    // STAT_SLOTS
     int stat_blocks = 0;
     double *h_stats = nullptr;                  // pinned host mirror of stats + time
+    float *h_stage = nullptr;                   // behind it, up to STAGE_CELLS: 8 N floats for mms_hfield_host
 
     FmmPlan *fmm = nullptr;
 
