@@ -397,14 +397,18 @@ int mms_ctx_create(const mms_grid *grid, const mms_params *params, const mms_sol
         const size_t N = (size_t)ctx->N;
         ctx->stat_blocks = (int)div_up(ctx->N, 256);
         {
-            // the allocations below, each padded to 256 bytes; without memory
-            // for them in one piece they are tried one by one
+            // The allocations below, each padded to 256 bytes, in one piece:
+            // 256 x 256 x 3 3.2 -> 0.56 ms a context.  Not where the piece would
+            // be mapped for itself and each of them (24 N bytes) is small enough for
+            // the driver's pool: 64 x 64 x 3 80 us against 410.  Without memory
+            // for the piece they are tried one by one.
             const size_t sizes[] = {4 * N, 4 * N, 4 * N, 12 * N, 12 * N, N, 24 * N, 24 * N, 24 * N, 24 * N, 24 * N,
                                     24 * N, TIME_SLOTS * 8, 4 * MMS_MAX_HEXT * 8, (size_t)ctx->stat_blocks * 64,
                                     STAT_SLOTS * 8};
             for (size_t b : sizes) ctx->arena_bytes += (b + 255) / 256 * 256;
             if (!solver || solver->kind == MMS_SOLVER_DIRECT) ctx->arena_bytes += direct_bytes(*grid);
-            if (cudaMalloc((void **)&ctx->arena, ctx->arena_bytes) != cudaSuccess) {
+            if ((ctx->arena_bytes <= 1 << 20 || 24 * N > 1 << 19) &&
+                cudaMalloc((void **)&ctx->arena, ctx->arena_bytes) != cudaSuccess) {
                 cudaGetLastError();
                 ctx->arena = nullptr;
             }
