@@ -409,8 +409,11 @@ __global__ void __launch_bounds__(512) k_p2m_row(const float *__restrict__ rho, 
 
 // k_p2m_row for grids of many leaf boxes: a CTA takes the 32 x 16 columns of
 // k_l2p_wide.  The charges are staged as [4 boxes of a row][cell], so that a
-// thread (4 boxes, one coefficient) has 16 sums from one weight (through L1,
-// where every CTA of the SM finds it) and one 16-byte broadcast a cell.  With
+// thread (4 boxes, one coefficient) has 4 products from one weight and one
+// 16-byte broadcast a cell; weights and operators stream in while the
+// predecessor finishes (read through L1 as they went: 82 us instead of 30 at
+// 1024 x 1024 x 3, leaf 8, P = 4, where k_p2m_row took 52; 512 x 512 x 3 at
+// leaf 4 115 -> 106 us a potential).  With
 // up the parents follow, thread per (parent, coefficient).  Per output the
 // arithmetic of p2m_dot and m2m_reduce, so the same bits.
 // Shared memory: charges [NB / 4][C][4], (up) the leaves' expansions [NB][NR],
@@ -677,14 +680,13 @@ __global__ void __launch_bounds__(32 * M2L_WARPS) k_m2l_split(const float *__res
         if (k0 + i < NB) Lt[k0 + i] = acc[i];
 }
 
-// M2L for low orders, all levels >= 2 in one launch: every operator block of
-// the 49 offset slots stays resident in shared memory (P <= 5).  CTA = 32
-// targets of one (level, parity class) x 8 warps; warp w takes offsets
-// w, w+8, w+16, w+24 of the class's 27; lane <-> target.  Each lane keeps its
-// source expansion and both parity blocks of its partial local in registers
-// and reads the operator rows as warp-uniform float2 broadcasts.  The 8 warps'
-// partials are summed in a fixed order in shared memory; the result is the
-// complete M2L local (one partial buffer).
+// M2L for low orders (P <= 5), all levels >= 2 in one launch: the operator
+// blocks of a parity class's 27 offsets stay resident in shared memory.  CTA =
+// 16 or 32 targets of one (level, parity class) at a time x 8 warps.  Each lane
+// has its target's source expansion and both parity blocks of its partial local
+// in registers and reads the operators as broadcasts.  The 8 warps' partials
+// are summed in a fixed order in shared memory; the result is the complete M2L
+// local (one partial buffer).
 constexpr int RES_WARPS = 8;
 constexpr int RES_TPI = 16;  // targets per resident-M2L item
 
@@ -2900,8 +2902,6 @@ static int l2p_up(const FmmPlan *pl) { return pl->d.L >= 3 && leaf_threads(pl->d
 static int p2m_up(const FmmPlan *pl) { return l2p_up(pl) && pl->d.NR <= 32; }
 // levels 2 and 3 share one launch each way (k_top_m2m / k_top_l2l: 16 KT <= 512 threads)
 static int top_two(const FmmPlan *pl) { return pl->d.NR <= 32 && !pl->far_fused; }
-// L2P also forms levels 2 .. L-2 of each CTA's ancestors (pmode 4): no L2L
-// launch at all between the M2L and L2P
 
 // k_l2p_wide and the L2L passes it needs, from the grid on where its CTAs of
 // 32 x 16 columns fill the chip.  A potential of P = 4 and 3 layers, k_l2p with
@@ -2914,6 +2914,8 @@ static int l2p_wide(const FmmPlan *pl)
     return l2p_up(pl) && f.L >= 4 && (f.s == 4 || f.s == 8) && f.Z <= 16 &&
            (long long)div_up(f.X, 32) * div_up(f.Y, 16) >= 240;
 }
+// else L2P also forms levels 2 .. L-2 of each CTA's ancestors (pmode 4): no L2L
+// launch at all between the M2L and L2P
 static int l2p_top(const FmmPlan *pl) { return l2p_up(pl) && pl->d.L >= 4 && !l2p_wide(pl); }
 
 template <int S, int R>
