@@ -1741,7 +1741,8 @@ __global__ void __launch_bounds__(512) k_l2p_wide(const float *__restrict__ near
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int x = bx0 * S + lane;
     const long long cell0 = ((long long)warp * f.Y + by0 * S) * f.X + x;
-    const int rows = x < f.X ? min(R * S, f.Y - by0 * S) : 0;  // rows of the grid in this lane's column
+    const bool act = warp < f.Z;  // (the others help with the locals)
+    const int rows = act && x < f.X ? min(R * S, f.Y - by0 * S) : 0;  // rows of the grid in this lane's column
     float acc[R * S];
 #pragma unroll
     for (int y = 0; y < R * S; y++) acc[y] = y < rows ? near[cell0 + (long long)y * f.X] : 0.f;
@@ -1787,6 +1788,7 @@ __global__ void __launch_bounds__(512) k_l2p_wide(const float *__restrict__ near
         Lb[k * LP + b] = v;
     }
     __syncthreads();
+    if (!act) return;
     const float *lb = Lb + lane / S;
     const float *vc = Vt + warp * S * S + lane % S;
 #pragma unroll 2
@@ -2926,8 +2928,10 @@ static int l2p_wide_launch(const FmmPlan *pl, const float *near, const float *Lg
     constexpr int BX = 32 / S, NB = BX * R, NP = NB / 4, GX = BX / 4;
     const size_t smem = (4 * ((size_t)f.NE * f.NE + (size_t)(f.NR - f.NE) * (f.NR - f.NE)) +
                          (size_t)f.NR * (NB + 1 + NP + GX)) * sizeof(float);
+    // a warp a layer; more of them, for the locals alone, where those are many
+    // (400 x 400 x 2, leaf 4, P = 8: 424 -> 370 us a potential)
     MMS_CUDA_TRY(launch_k(k_l2p_wide<S, R>, dim3(div_up(f.X, 32), div_up(f.Y, R * S)),
-                          dim3(32 * f.Z), smem, st, near, (const float *)(pl->Lpart + pl->lev_off[f.L] * f.NR),
+                          dim3(std::max(32 * f.Z, std::min(256, (NB * f.NR / 16 + 31) / 32 * 32))), smem, st, near, (const float *)(pl->Lpart + pl->lev_off[f.L] * f.NR),
                           (const float *)pl->Tl2l, (const float *)pl->Vt, phi, f, pl->nbox_total * f.NR, nsplit, Lgp, Lpp,
                           nnear, near_stride));
     return MMS_OK;
