@@ -3018,7 +3018,11 @@ static int p2m_launch(mms_ctx *ctx, const float *rho, const DivSrc *dv)
         block(up ? (PB / 2) * 4 * KT : std::min(512, ((PB * f.NR + 31) / 32) * 32));
     const long long off_par = up ? pl->lev_off[f.L - 1] : 0LL;
     const DivSrc d0 = dv ? *dv : DivSrc{};
-    if (l2p_wide(pl)) {
+    // (not for long expansions of many cells: the weights are read through L1
+    // then; 512 x 512 x 6, leaf 8, P = 5: 353 us a potential with k_p2m_row, 380
+    // with the wide form, but 512 x 512 x 8 at P = 4 529 against 509 and 1024 x
+    // 1024 x 3 at P = 6 448 against 411)
+    if (l2p_wide(pl) && !(f.NR > 32 && f.C > 256)) {
         const int NB = 32 / f.s * (16 / f.s);
         const int wide_w = (size_t)f.C * f.NR * sizeof(float) <= 40 * 1024;
         const size_t wide_smem = ((size_t)NB * (f.C + (up ? f.NR : 0) + (f.s == 8 ? 4 * f.NR : 0)) +
