@@ -10,7 +10,6 @@ using namespace mmsconv;
 
 namespace {
 
-constexpr size_t SMEM_MAX = 200 * 1024;   // per CTA
 constexpr int ROW_PAIRS = 4;              // row pairs per CTA at most: small grids need the CTAs
 constexpr int MAX_THREADS = 512;          // threads of a row or column CTA
 
@@ -190,17 +189,6 @@ int conv_build_tables(ConvDev &c, void *tab, double *scratch, double dx, double 
     return MMS_OK;
 }
 
-// raises a kernel's dynamic shared-memory limit (never lowers it: the limit is
-// shared by every context and ensemble)
-int conv_raise_smem(const void *kernel, size_t bytes)
-{
-    cudaFuncAttributes fa{};
-    MMS_CUDA_TRY(cudaFuncGetAttributes(&fa, kernel));
-    if ((size_t)fa.maxDynamicSharedSizeBytes < bytes)
-        MMS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    return MMS_OK;
-}
-
 }  // namespace mmsconv
 
 struct ConvPlan {
@@ -243,11 +231,11 @@ int conv_plan_create(mms_ctx *ctx, ConvPlan **out)
     int st = conv_build_tables(c, (char *)pl.mem + first, (double *)pl.mem, ctx->g.dx, ctx->g.dy, ctx->g.dz,
                                ctx->stream, &ctx->launches);
     with_plan(pl.g.px.id, [&](auto p) {
-        if (!st) st = conv_raise_smem((const void *)k_conv_rows<decltype(p)>, smem);
-        if (!st) st = conv_raise_smem((const void *)k_conv_back<decltype(p)>, smem);
+        if (!st) st = allow_smem((const void *)k_conv_rows<decltype(p)>);
+        if (!st) st = allow_smem((const void *)k_conv_back<decltype(p)>);
     });
     with_plan(pl.g.py.id, [&](auto p) {
-        if (!st) st = conv_raise_smem((const void *)k_conv_columns<decltype(p)>, smem);
+        if (!st) st = allow_smem((const void *)k_conv_columns<decltype(p)>);
     });
     if (st) {
         ctx_free(ctx, pl.mem);

@@ -323,7 +323,6 @@ size_t conv_table_scratch(const ConvDev &c);
 // past the launches
 int conv_build_tables(ConvDev &c, void *tab, double *scratch, double dx, double dy, double dz, cudaStream_t st,
                       int64_t *launches);
-int conv_raise_smem(const void *kernel, size_t bytes);
 
 // One Stockham pass of nf transforms, one butterfly per thread (nf n / R <=
 // blockDim): ld(f) gives a reader of transform f's elements, st(f) a writer.

@@ -206,7 +206,6 @@ size_t direct_smem_bytes(int X)
 // per two 16-byte reads as in k_direct; a row's FP32 sum is added to FP64 sums,
 // and the S partial sums of a target are added in a fixed order.
 constexpr int SMALL_THREADS = 512;
-constexpr size_t SMALL_SMEM = 200 * 1024;
 
 struct SmallShape {
     int X, Y, Z, rows;   // rows = Y Z
@@ -340,7 +339,7 @@ bool small_shape(const mms_grid &g, SmallShape &s)
     s.tiles = (all + s.segs - 1) / s.segs;
     s.segs = (all + s.tiles - 1) / s.tiles;
     s.S = std::max(1, std::min(s.rows, SMALL_THREADS / s.tiles));
-    return s.tiles <= SMALL_THREADS && small_smem(s) <= SMALL_SMEM;
+    return s.tiles <= SMALL_THREADS && small_smem(s) <= SMEM_MAX;
 }
 
 }  // namespace
@@ -371,9 +370,9 @@ int direct_prepare(mms_ctx *ctx)
         k_build_gsmall<<<div_up((long long)s.rows * s.pitch, 256), 256, 0, ctx->stream>>>(ctx->gsmall, s, ctx->g.dx,
                                                                                       ctx->g.dy, ctx->g.dz);
         MMS_LAUNCH_CHECK(ctx);
-        MMS_TRY(mmsconv::conv_raise_smem((const void *)k_direct_small<0>, SMALL_SMEM));
-        MMS_TRY(mmsconv::conv_raise_smem((const void *)k_direct_small<1>, SMALL_SMEM));
-        MMS_TRY(mmsconv::conv_raise_smem((const void *)k_direct_small<2>, SMALL_SMEM));
+        MMS_TRY(allow_smem((const void *)k_direct_small<0>));
+        MMS_TRY(allow_smem((const void *)k_direct_small<1>));
+        MMS_TRY(allow_smem((const void *)k_direct_small<2>));
         if (ctx->N <= SMALL_STEP_MAX) return MMS_OK;
     }
     MMS_TRY(conv_plan_create(ctx, &ctx->conv));

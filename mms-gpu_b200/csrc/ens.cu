@@ -558,14 +558,7 @@ int ens_set_shape(mms_ens *e, int ew, int qrows)
     e->ew = ew;
     e->qrows = qrows;
     e->direct_smem = direct_smem_for(e->ts, qrows);
-    {
-        // the limit is per kernel and shared by every ensemble: only ever raise it
-        cudaFuncAttributes fa{};
-        MMS_CUDA_TRY(cudaFuncGetAttributes(&fa, k_ens_direct));
-        if ((size_t)fa.maxDynamicSharedSizeBytes < e->direct_smem)
-            MMS_CUDA_TRY(cudaFuncSetAttribute(k_ens_direct, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)e->direct_smem));
-    }
+    MMS_TRY(allow_smem((const void *)k_ens_direct));
     int dev = 0, sms = 0, per = 0;
     MMS_CUDA_TRY(cudaGetDevice(&dev));
     MMS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -709,9 +702,9 @@ int ens_conv_prepare(mms_ens *e)
     MMS_CUDA_TRY(cudaMemcpyAsync(e->row_items, items.data(), items.size() * sizeof(ConvItem), cudaMemcpyHostToDevice,
                                  e->stream));
     MMS_CUDA_TRY(cudaStreamSynchronize(e->stream));
-    MMS_TRY(conv_raise_smem((const void *)k_ens_rows, smem));
-    MMS_TRY(conv_raise_smem((const void *)k_ens_columns, smem));
-    MMS_TRY(conv_raise_smem((const void *)k_ens_back, smem));
+    MMS_TRY(allow_smem((const void *)k_ens_rows));
+    MMS_TRY(allow_smem((const void *)k_ens_columns));
+    MMS_TRY(allow_smem((const void *)k_ens_back));
     return MMS_OK;
 }
 
@@ -775,7 +768,7 @@ int mms_ens_create(const mms_ens_instance *inst, int n, double dx, double dy, do
     ts.C = ts.Xm + 3;
     ts.pitch = 2 * ts.Xm + 8;
     const size_t smem = direct_smem_for(ts, QROWS_MAX);
-    if (smem > 200 * 1024) {
+    if (smem > SMEM_MAX) {
         mms_set_error("mms_ens_create: the shared kernel table (%zu B) exceeds 200 KiB; largest instance too big",
                       smem);
         return MMS_ERR_ARG;

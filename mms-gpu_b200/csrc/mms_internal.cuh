@@ -309,4 +309,16 @@ inline void ctx_free(mms_ctx *ctx, void *p)
     if (p && !(ctx->arena && (char *)p >= ctx->arena && (char *)p < ctx->arena + ctx->arena_bytes)) cudaFree(p);
 }
 
+// Dynamic shared memory per CTA of the kernels whose need depends on the grid.
+// A kernel's limit is one for the whole process, shared by every context,
+// ensemble and host thread: it is always set to this same value, so that no
+// caller lowers it below another's need (reading it first and raising it where
+// it is too small let two threads set their own needs in the wrong order).
+constexpr size_t SMEM_MAX = 200 * 1024;
+inline int allow_smem(const void *kernel)
+{
+    MMS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+    return MMS_OK;
+}
+
 static inline unsigned div_up(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
