@@ -231,11 +231,11 @@ int conv_plan_create(mms_ctx *ctx, ConvPlan **out)
     int st = conv_build_tables(c, (char *)pl.mem + first, (double *)pl.mem, ctx->g.dx, ctx->g.dy, ctx->g.dz,
                                ctx->stream, &ctx->launches);
     with_plan(pl.g.px.id, [&](auto p) {
-        if (!st) st = allow_smem((const void *)k_conv_rows<decltype(p)>);
-        if (!st) st = allow_smem((const void *)k_conv_back<decltype(p)>);
+        if (!st) st = allow_smem((const void *)k_conv_rows<decltype(p)>, smem);
+        if (!st) st = allow_smem((const void *)k_conv_back<decltype(p)>, smem);
     });
     with_plan(pl.g.py.id, [&](auto p) {
-        if (!st) st = allow_smem((const void *)k_conv_columns<decltype(p)>);
+        if (!st) st = allow_smem((const void *)k_conv_columns<decltype(p)>, smem);
     });
     if (st) {
         ctx_free(ctx, pl.mem);

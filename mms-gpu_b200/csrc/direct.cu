@@ -370,9 +370,9 @@ int direct_prepare(mms_ctx *ctx)
         k_build_gsmall<<<div_up((long long)s.rows * s.pitch, 256), 256, 0, ctx->stream>>>(ctx->gsmall, s, ctx->g.dx,
                                                                                       ctx->g.dy, ctx->g.dz);
         MMS_LAUNCH_CHECK(ctx);
-        MMS_TRY(allow_smem((const void *)k_direct_small<0>));
-        MMS_TRY(allow_smem((const void *)k_direct_small<1>));
-        MMS_TRY(allow_smem((const void *)k_direct_small<2>));
+        MMS_TRY(allow_smem((const void *)k_direct_small<0>, small_smem(s)));
+        MMS_TRY(allow_smem((const void *)k_direct_small<1>, small_smem(s)));
+        MMS_TRY(allow_smem((const void *)k_direct_small<2>, small_smem(s)));
         if (ctx->N <= SMALL_STEP_MAX) return MMS_OK;
     }
     MMS_TRY(conv_plan_create(ctx, &ctx->conv));

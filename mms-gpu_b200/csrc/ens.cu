@@ -558,7 +558,7 @@ int ens_set_shape(mms_ens *e, int ew, int qrows)
     e->ew = ew;
     e->qrows = qrows;
     e->direct_smem = direct_smem_for(e->ts, qrows);
-    MMS_TRY(allow_smem((const void *)k_ens_direct));
+    MMS_TRY(allow_smem((const void *)k_ens_direct, e->direct_smem));
     int dev = 0, sms = 0, per = 0;
     MMS_CUDA_TRY(cudaGetDevice(&dev));
     MMS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -702,9 +702,9 @@ int ens_conv_prepare(mms_ens *e)
     MMS_CUDA_TRY(cudaMemcpyAsync(e->row_items, items.data(), items.size() * sizeof(ConvItem), cudaMemcpyHostToDevice,
                                  e->stream));
     MMS_CUDA_TRY(cudaStreamSynchronize(e->stream));
-    MMS_TRY(allow_smem((const void *)k_ens_rows));
-    MMS_TRY(allow_smem((const void *)k_ens_columns));
-    MMS_TRY(allow_smem((const void *)k_ens_back));
+    MMS_TRY(allow_smem((const void *)k_ens_rows, smem));
+    MMS_TRY(allow_smem((const void *)k_ens_columns, smem));
+    MMS_TRY(allow_smem((const void *)k_ens_back, smem));
     return MMS_OK;
 }
 

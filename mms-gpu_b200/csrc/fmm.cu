@@ -2243,25 +2243,16 @@ size_t l2p_smem(const FmmDev &f)
 
 int leaf_set_smem(const FmmDev &f)
 {
-    const int a = (int)p2p_smem(f), b = (int)l2p_smem(f);
-    cudaError_t e = cudaSuccess;
-#define X(S_, B_)                                                                                    \
-    if (f.s == S_ && a > 48 * 1024) {                                                                \
-        e = cudaFuncSetAttribute(k_p2p<S_, B_, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, a);   \
-        if (e == cudaSuccess)                                                                        \
-            e = cudaFuncSetAttribute(k_p2p<S_, B_, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, a); \
-    }                                                                                                \
-    if (f.s == S_ && e == cudaSuccess && b > 48 * 1024) {                                            \
-        e = cudaFuncSetAttribute(k_l2p<S_, B_, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);   \
-        if (e == cudaSuccess)                                                                        \
-            e = cudaFuncSetAttribute(k_l2p<S_, B_, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, b); \
+    const size_t a = p2p_smem(f), b = l2p_smem(f);
+#define X(S_, B_)                                                   \
+    if (f.s == S_) {                                                \
+        MMS_TRY(allow_smem((const void *)k_p2p<S_, B_, 1>, a));     \
+        MMS_TRY(allow_smem((const void *)k_p2p<S_, B_, 3>, a));     \
+        MMS_TRY(allow_smem((const void *)k_l2p<S_, B_, 1>, b));     \
+        MMS_TRY(allow_smem((const void *)k_l2p<S_, B_, 3>, b));     \
     }
     MMS_LEAF_CASES(X)
 #undef X
-    if (e != cudaSuccess) {
-        mms_set_error("leaf kernel shared memory (%d / %d B): %s", a, b, cudaGetErrorString(e));
-        return MMS_ERR_ARG;
-    }
     return MMS_OK;
 }
 
@@ -2708,8 +2699,7 @@ int fmm_plan_create(mms_ctx *ctx)
     MMS_LAUNCH_CHECK(ctx);
     pl->lev_dev = lev_dev;
     const size_t m2ls_smem = ((size_t)NBmax * KPmax + 32 * (size_t)(NBmax | 1)) * sizeof(float);
-    if (m2ls_smem > 48 * 1024)
-        MMS_CUDA_TRY(cudaFuncSetAttribute(k_m2l_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m2ls_smem));
+    MMS_TRY(allow_smem((const void *)k_m2l_split, m2ls_smem));
     if (pl->m2l_resident) MMS_TRY(m2l_res_prepare(NR, f.NE));
     if (pl->m2l_resident && NR <= 30 && leaf_threads(f) > 0 && f.L >= 2 && ctx->s.far_mode == 1)
         MMS_TRY(far_prepare(ctx, pl));
@@ -2729,11 +2719,8 @@ int fmm_plan_create(mms_ctx *ctx)
         const size_t tsz = 4 * cstride;
         const int KT = ((NR + 31) / 32) * 32;
         const size_t a1 = (tsz + 4 * (size_t)NR + 4 * (size_t)KT) * sizeof(float), a2 = (tsz + (size_t)NR) * sizeof(float);
-        if (a1 > 48 * 1024)
-            MMS_CUDA_TRY(cudaFuncSetAttribute(k_m2m_c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a1));
-        if (a2 > 48 * 1024)
-            MMS_CUDA_TRY(cudaFuncSetAttribute(k_l2l_c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a2));
-
+        MMS_TRY(allow_smem((const void *)k_m2m_c, a1));
+        MMS_TRY(allow_smem((const void *)k_l2l_c, a2));
     }
     if (leaf_threads(f) > 0) MMS_TRY(leaf_set_smem(f));
     MMS_TRY(fmm_set_carveout());
@@ -3205,8 +3192,7 @@ int far_prepare(mms_ctx *ctx, FmmPlan *pl)
         scratch = far_scratch<a, c>(f.C);                                                            \
         pl->far_smem = (size_t)(57 * OSZ + scratch) * sizeof(float);                                 \
         if (pl->far_smem > 227 * 1024) return MMS_OK;                                                \
-        MMS_CUDA_TRY(cudaFuncSetAttribute(k_far<a, c>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
-                                          (int)pl->far_smem));                                      \
+        MMS_TRY(allow_smem((const void *)k_far<a, c>, pl->far_smem));                                 \
         MMS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_far<a, c>, 32 * RES_WARPS, \
                                                                    pl->far_smem));                   \
     }

@@ -309,15 +309,24 @@ inline void ctx_free(mms_ctx *ctx, void *p)
     if (p && !(ctx->arena && (char *)p >= ctx->arena && (char *)p < ctx->arena + ctx->arena_bytes)) cudaFree(p);
 }
 
-// Dynamic shared memory per CTA of the kernels whose need depends on the grid.
-// A kernel's limit is one for the whole process, shared by every context,
-// ensemble and host thread: it is always set to this same value, so that no
-// caller lowers it below another's need (reading it first and raising it where
-// it is too small let two threads set their own needs in the wrong order).
-constexpr size_t SMEM_MAX = 200 * 1024;
-inline int allow_smem(const void *kernel)
+// Dynamic shared memory of a kernel whose need depends on the grid or the
+// order.  The limit is one for the whole process, shared by every context,
+// ensemble and host thread: it is always set to all that a CTA can have, so that
+// no caller lowers it below another's need (set to each plan's own need, a
+// plan of order 8 left one of order 9 without its M2M; raised where it read too
+// small, two threads could set their needs in the wrong order).
+constexpr size_t SMEM_CTA = 227 * 1024;  // static and dynamic
+constexpr size_t SMEM_MAX = 200 * 1024;  // what the kernels of other solvers than the FMM ask for at most
+inline int allow_smem(const void *kernel, size_t need)
 {
-    MMS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX));
+    cudaFuncAttributes fa{};
+    MMS_CUDA_TRY(cudaFuncGetAttributes(&fa, kernel));
+    const size_t most = SMEM_CTA - fa.sharedSizeBytes;
+    if (need > most) {
+        mms_set_error("a kernel needs %zu bytes of shared memory, a CTA has %zu", need, most);
+        return MMS_ERR_ARG;
+    }
+    MMS_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
     return MMS_OK;
 }
 

@@ -50,3 +50,28 @@ def test_contexts_created_by_several_threads(cuda, lib):
     r = subprocess.run([sys.executable, "-c", THREADS, ROOT + "/mms-gpu_b200"], capture_output=True, text=True,
                        timeout=300)
     assert r.returncode == 0 and "done" in r.stdout, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(m2l_mode=1), dict(near_mode=1)])
+@pytest.mark.parametrize("first,second", [((9, 8, 3), (8, 8, 3)), ((9, 4, 3), (8, 4, 3)), ((9, 8, 2), (9, 8, 1)),
+                                          ((8, 8, 8), (7, 8, 8)), ((3, 8, 16), (3, 8, 15))])
+def test_a_smaller_plan_leaves_a_larger_one_its_kernels(cuda, lib, first, second, kw):
+    """two FMM contexts (order, leaf side, layers) live together: the second
+    one needs less shared memory of the same kernels, and the first one's
+    potential is that from before"""
+    import mmsb200
+    torch = cuda
+
+    def context(P, leaf, Z):
+        return mmsb200.Context(mmsb200.Grid(64, 64, Z, 5e-9, 5e-9, 5e-9), mmsb200.make_params(),
+                               mmsb200.make_solver(mmsb200.SOLVER_FMM, P, leaf, **kw))
+
+    rho = torch.randn(first[2], 64, 64, device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+    before, after = torch.empty_like(rho), torch.empty_like(rho)
+    with context(*first) as a:
+        a.potential_dev(rho, before)
+        a.sync()
+        with context(*second):
+            a.potential_dev(rho, after)
+            a.sync()
+    assert torch.equal(before, after)
