@@ -870,7 +870,12 @@ int gradient(mms_farnet *n, const float *u, const float *far, const float *nrm2,
     MMS_CUDA_TRY(cudaMemcpyAsync(hr, n->res, sizeof(FarnetResult), cudaMemcpyDeviceToHost, 0));
     if (grad) MMS_CUDA_TRY(cudaMemcpyAsync(hg, n->g, gbytes, cudaMemcpyDeviceToHost, 0));
     MMS_CUDA_TRY(cudaStreamSynchronize(0));
-    if (hr->err) return umma_check_error();
+    if (hr->err) {
+        // (the word is the device's: another caller may have read and cleared it since)
+        MMS_TRY(umma_check_error());
+        mms_set_error("farnet: an mbarrier wait of a tensor-core GEMM timed out");
+        return MMS_ERR_CUDA;
+    }
     if (loss) *loss = hr->loss;
     if (grad) memcpy(grad, hg, gbytes);
     return MMS_OK;

@@ -441,3 +441,41 @@ def test_gradient_at_the_edges_of_its_levels(cuda, lib, oracle_mod, dims, batch)
     assert abs(loss - lref) <= 1e-5 * lref, (loss, lref)
     assert rel_l2(g, gref) < 1e-4
     assert np.array_equal(g, again)
+
+
+def test_gradient_never_succeeds_without_its_results(cuda, lib):
+    """The GEMM core's error word is one for the device: a gradient that found
+    it set is an error also when somebody else has cleared the word since.  The
+    word is set by hand here and cleared by another stream at many moments
+    around the end of the call."""
+    import ctypes
+    import torch
+    import mmsb200
+    f = getattr(lib, "_Z15umma_error_wordv")
+    f.restype = ctypes.c_void_p
+
+    class Word:
+        __cuda_array_interface__ = {"shape": (1,), "typestr": "<i4", "data": (f(), False), "version": 3}
+
+    word, side = torch.as_tensor(Word(), device="cuda"), torch.cuda.Stream()
+    u = torch.randn(1, 3, 33, 33, device="cuda")
+    nrm = (u ** 2).sum().reshape(1)
+    seen = 0
+    with mmsb200.FarNet(33, 33, batch=1) as net:
+        net.set_weights(_weights())
+        for cycles in range(100_000, 900_000, 2_000):
+            torch.cuda.synchronize()
+            word.fill_(1)
+            torch.cuda.synchronize()
+            with torch.cuda.stream(side):
+                torch.cuda._sleep(cycles)
+                word.zero_()
+            g, loss = np.full(net.num_params(), np.nan, np.float32), ctypes.c_double(np.nan)
+            st = lib.mms_farnet_gradient(net.h, u.data_ptr(), u.data_ptr(), nrm.data_ptr(), 1, g.ctypes.data,
+                                         ctypes.byref(loss))
+            seen += st == 0
+            assert st != 0 or (np.isfinite(loss.value) and np.isfinite(g).all()), cycles
+    torch.cuda.synchronize()
+    word.zero_()
+    torch.cuda.synchronize()
+    assert 0 < seen < 400  # the word was found set by some calls and clear by others
