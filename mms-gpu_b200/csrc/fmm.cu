@@ -24,6 +24,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include <cuda.h>
@@ -1715,6 +1716,12 @@ __global__ void __launch_bounds__(512) k_l2p(const float *__restrict__ near, con
 // above come from L2L passes.  k_l2p is made for the shortest chain and bound by
 // its ancestors' serial sums and by partial lines here: 1024 x 1024 x 3, leaf 8,
 // P = 4: 115 us, this 34 us and 9 us of L2L passes.
+// The terms go onto the near field in groups (8 coefficients at leaf side 4, 4 at
+// 8: more registers cost CTAs there): one after the other they were a longer FP32
+// chain than k_l2p's three, and the potential's error against the FP64
+// restatement grew by up to 0.08 % (P = 6, leaf 4: 3.7858e-6 for 3.7827e-6; now
+// 3.7816e-6).  Potentials, one chain against the groups: 1024 x 1024 x 3, leaf 8,
+// P = 4 172.0 us and 172.5; 400 x 400 x 2, leaf 4, P = 8 369 and 355.
 template <int S, int R>
 __global__ void __launch_bounds__(512) k_l2p_wide(const float *__restrict__ near, const float *__restrict__ Lpart_leaf,
                                                   const float *__restrict__ Tl2l, const float *__restrict__ Vt,
@@ -1791,18 +1798,37 @@ __global__ void __launch_bounds__(512) k_l2p_wide(const float *__restrict__ near
     if (!act) return;
     const float *lb = Lb + lane / S;
     const float *vc = Vt + warp * S * S + lane % S;
-#pragma unroll 2
-    for (int k = 0; k < NR; k++) {
-        float l[R];
+    // the products of G coefficients are added up by themselves first
+    auto add = [&](auto g, int k) {
+        constexpr int G = decltype(g)::value;
+        float l[G][R];
 #pragma unroll
-        for (int r = 0; r < R; r++) l[r] = lb[k * LP + r * BX];
+        for (int q = 0; q < G; q++)
+#pragma unroll
+            for (int r = 0; r < R; r++) l[q][r] = lb[(k + q) * LP + r * BX];
 #pragma unroll
         for (int y = 0; y < S; y++) {
-            const float v = __ldg(vc + (long long)k * f.C + y * S);
+            float v[G];
 #pragma unroll
-            for (int r = 0; r < R; r++) acc[r * S + y] = fmaf(v, l[r], acc[r * S + y]);
+            for (int q = 0; q < G; q++) v[q] = __ldg(vc + (long long)(k + q) * f.C + y * S);
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                float t = v[0] * l[0][r];
+#pragma unroll
+                for (int q = 1; q < G; q++) t = fmaf(v[q], l[q][r], t);
+                acc[r * S + y] += t;
+            }
         }
+    };
+    constexpr int G = S == 4 ? 8 : 4;
+    int k = 0;
+#pragma unroll 1
+    for (; k + G <= NR; k += G) add(std::integral_constant<int, G>{}, k);
+    if (k + 4 <= NR) {  // (G = 8)
+        add(std::integral_constant<int, 4>{}, k);
+        k += 4;
     }
+    if (k < NR) add(std::integral_constant<int, 2>{}, k);  // NR is even
 #pragma unroll
     for (int y = 0; y < R * S; y++)
         if (y < rows) phi[cell0 + (long long)y * f.X] = acc[y];
