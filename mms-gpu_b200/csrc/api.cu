@@ -179,6 +179,17 @@ void drop_graph(mms_ctx *ctx)
     ctx->graph_kernels = 0;
 }
 
+// rho = div M of FP32 M and its potential by the FMM or the network.  rho may be
+// the caller's: whatever becomes of the potential, no later call may take the
+// charges' BF16 split for that of rho's next contents
+int charge_and_potential(mms_ctx *ctx, const float *M, float *rho, float *phi)
+{
+    MMS_TRY(launch_divergence_aos(ctx, M, rho, true));
+    const int st = launch_potential(ctx, rho, phi);
+    fmm_split_written(ctx, nullptr);
+    return st;
+}
+
 // potential of the state M into ctx->phi (rho = div M into ctx->rho)
 int eval_state_potential(mms_ctx *ctx, const double *Mst)
 {
@@ -598,9 +609,7 @@ int mms_hfield_dev(mms_ctx *ctx, const float *M, float *H, float *charge, float 
     if (ctx->p.demag && ctx->s.kind == MMS_SOLVER_DIRECT) {
         MMS_TRY(launch_potential_direct_aos(ctx, M, charge, phi));
     } else if (ctx->p.demag) {
-        MMS_TRY(launch_divergence_aos(ctx, M, rho, true));
-        MMS_TRY(launch_potential(ctx, rho, phi));
-        fmm_split_written(ctx, nullptr);
+        MMS_TRY(charge_and_potential(ctx, M, rho, phi));
     }
     MMS_TRY(launch_hfield_aos(ctx, M, phi, t, H));
     if (!potential) ctx->phi_valid = false;  // ctx->phi no longer holds the state's potential
@@ -651,9 +660,7 @@ int mms_hfield_host(mms_ctx *ctx, const float *M, float *H, float *charge, float
     if (ctx->p.demag && ctx->s.kind == MMS_SOLVER_DIRECT) {
         MMS_TRY(launch_potential_direct_aos(ctx, ctx->vecA, charge ? ctx->rho : nullptr, ctx->phi));
     } else if (ctx->p.demag) {
-        MMS_TRY(launch_divergence_aos(ctx, ctx->vecA, ctx->rho, true));
-        MMS_TRY(launch_potential(ctx, ctx->rho, ctx->phi));
-        fmm_split_written(ctx, nullptr);
+        MMS_TRY(charge_and_potential(ctx, ctx->vecA, ctx->rho, ctx->phi));
     }
     MMS_TRY(launch_hfield_aos(ctx, ctx->vecA, ctx->phi, t, ctx->vecB));
     ctx->phi_valid = false;

@@ -479,3 +479,31 @@ def test_gradient_never_succeeds_without_its_results(cuda, lib):
     word.zero_()
     torch.cuda.synchronize()
     assert 0 < seen < 400  # the word was found set by some calls and clear by others
+
+
+def test_a_field_that_failed_leaves_no_charges_behind(cuda, lib):
+    """A field call on a plan made anew, whose weights are not bound yet, fails after
+    it formed the charges (and their BF16 split for the near field) in the
+    caller's array.  A later potential of other contents of that array is theirs:
+    the bits of the same charges elsewhere."""
+    import torch
+    import mmsb200
+    gen = torch.Generator("cuda").manual_seed(5)
+    M = torch.randn(3, 64, 64, 3, device="cuda", generator=gen)
+    q, phi, ref = (torch.empty(3, 64, 64, device="cuda") for _ in range(3))
+    H = torch.empty_like(M)
+    with mmsb200.Context(mmsb200.Grid(64, 64, 3, 5e-9, 5e-9, 5e-9), mmsb200.make_params(),
+                         mmsb200.make_solver(mmsb200.SOLVER_SURROGATE, 6, 8)) as ctx:
+        ctx.set_surrogate(_weights())
+        ctx.set_solver(mmsb200.make_solver(mmsb200.SOLVER_SURROGATE, 6, 8))
+        with pytest.raises(mmsb200.MmsError):
+            ctx.hfield_dev(M, H, q, phi)
+        ctx.set_surrogate(_weights())
+        ctx.sync()
+        q.normal_(generator=gen)
+        other = q.clone()
+        torch.cuda.synchronize()
+        ctx.potential_dev(q, phi)
+        ctx.potential_dev(other, ref)
+        ctx.sync()
+    assert torch.equal(phi, ref)
