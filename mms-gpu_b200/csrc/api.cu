@@ -411,8 +411,11 @@ int mms_ctx_create(const mms_grid *grid, const mms_params *params, const mms_sol
             // The allocations below, each padded to 256 bytes, in one piece:
             // 256 x 256 x 3 3.2 -> 0.56 ms a context.  Not where the piece would
             // be mapped for itself and each of them (24 N bytes) is small enough for
-            // the driver's pool: 64 x 64 x 3 80 us against 410.  Without memory
-            // for the piece they are tried one by one.
+            // the driver's pool: 64 x 64 x 3 80 us against 410.  FMM contexts (P = 4,
+            // leaf 8), plan and tables among it, one by one and in one piece: 256 x
+            // 256 x 3 16.7 and 14.4 ms, 512 x 512 x 3 17.9 and 15.0, 1024 x 1024 x 3
+            // 19.2 and 16.5, 1448 x 1448 x 3 22.0 and 19.6.  Without memory for the
+            // piece they are tried one by one.
             const size_t sizes[] = {4 * N, 4 * N, 4 * N, 12 * N, 12 * N, N, 24 * N, 24 * N, 24 * N, 24 * N, 24 * N,
                                     24 * N, TIME_SLOTS * 8, 4 * MMS_MAX_HEXT * 8, (size_t)ctx->stat_blocks * 64,
                                     STAT_SLOTS * 8};

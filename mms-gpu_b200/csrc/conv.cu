@@ -114,11 +114,12 @@ __global__ void __launch_bounds__(MAX_THREADS) k_conv_back(ConvDev c, const doub
     extern __shared__ __align__(16) double2 cbuf[];
     pdl_begin();
     const int np = c.Z * ((c.Y + 1) >> 1), p0 = blockIdx.x * c.fb, cs = c.cs, X = c.X, Y = c.Y;
-    rows_back<row_pairs<PL>(MAX_THREADS, ROW_PAIRS)>(PL{}, c, cbuf, p0, min(c.fb, np - p0), [=](int k) { return store + (long long)k * cs; },
-              [=](int z, int y) {
-                  float *r = phi + ((long long)z * Y + y) * X;
-                  return [=](int x, float v) { r[x] = v; };
-              });
+    rows_back<row_pairs<PL>(MAX_THREADS, ROW_PAIRS)>(PL{}, c, cbuf, p0, min(c.fb, np - p0),
+                                                     [=](int k) { return store + (long long)k * cs; },
+                                                     [=](int z, int y) {
+                                                         float *r = phi + ((long long)z * Y + y) * X;
+                                                         return [=](int x, float v) { r[x] = v; };
+                                                     });
 }
 
 }  // namespace
@@ -218,7 +219,11 @@ size_t conv_plan_bytes(const mms_grid &g)
 
 // The convolution plan of a context's grid; *out stays NULL (and MMS_OK) where
 // the pair sum serves the grid: more than ZMAX layers, rows or columns beyond
-// the transforms' length, or no memory for the column store.
+// the transforms' length (2,048 cells), no memory for the column store, or
+// columns that a CTA cannot hold: all layers of one are transformed together,
+// 16 bytes for each of Z padded transforms, in at most 200 KB.  Beyond 512 cells
+// along y that means fewer layers: 7 to 768 cells, 5 to 1,024, 2 to 2,048 (along
+// x rows have no such limit: lay the longer side there).
 int conv_plan_create(mms_ctx *ctx, ConvPlan **out)
 {
     *out = nullptr;

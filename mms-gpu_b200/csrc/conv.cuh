@@ -14,7 +14,7 @@
 //   rows    two half spectra are joined into one complex transform back,
 //           phi is rounded to FP32
 //
-// Transforms are Stockham passes of radix 3, 4, 5, 8 or 16, one butterfly per
+// Transforms are Stockham passes of radix 3, 4, 5, 6, 8, 10, 12 or 16, one butterfly per
 // thread and pass, in place in shared memory (every thread reads its inputs
 // into registers, the CTA synchronises, then every thread writes), the first
 // pass reading its source and the last writing its destination where that can
@@ -23,9 +23,10 @@
 // long as the butterflies).  The inverse is the forward transform with real
 // and imaginary parts exchanged before and after.
 //
-// This header is the form with the columns in device memory, a launch per
-// pass; conv_sim.cu keeps those of small grids in the shared memory of a
-// cluster of CTAs.
+// The columns are kept in device memory, a launch per pass (conv.cu for a
+// context's grid, ens.cu for all instances of an ensemble).
+//
+// A charge that is not finite leaves no value of the potential finite.
 #pragma once
 
 #include "mms_internal.cuh"

@@ -2,8 +2,9 @@
 // reference's calc_potential_exact, fmm_calc.cu:412-461, and its GPU kernel
 // potential_calc.cu:18-116).  Contexts evaluate it as a convolution (conv.cu)
 // where the grid has a plan, small grids in one launch (k_direct_small); the
-// O(N^2) pair sum k_direct is for the other grids (more than 8 layers, rows or
-// columns beyond the transforms) and for the allocation-free entry point.
+// O(N^2) pair sum k_direct is for the other grids (more than 8 layers, fewer
+// where the columns are longer than 512 cells, see conv_plan_create; no memory for
+// the convolution) and for the allocation-free entry point.
 //
 // B200 design of k_direct.  On a regular grid 1/|r_i - r_j| depends only on the integer
 // offset, so the sum is a 3-D aperiodic convolution.  A table

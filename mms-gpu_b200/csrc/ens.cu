@@ -179,7 +179,8 @@ __global__ void __launch_bounds__(ETPB) k_ens_stage(const float *__restrict__ ph
         M[gi + N] = n1;
         M[gi + 2 * N] = n2;
     }
-  }  if (stage != 3) return;
+  }
+  if (stage != 3) return;
   __syncthreads();
   if (threadIdx.x == 0) {
       unsigned *ctr = reinterpret_cast<unsigned *>(tstate + TIME_CTR);
@@ -277,11 +278,12 @@ __global__ void __launch_bounds__(CONV_THREADS) k_ens_back(const EnsConv *__rest
     float *ph = phi + in.off;
     const int cs = c.cs, X = c.X, Y = c.Y, np = c.Z * ((c.Y + 1) >> 1) - it.first;
     mmsconv::with_batch_plan(c.px.id, [&](auto pl) {
-        mmsconv::rows_back<mmsconv::row_pairs<decltype(pl)>(CONV_THREADS, CONV_PAIRS)>(pl, c, cbuf, it.first, min(c.fb, np), [=](int k) { return st + k * cs; },
-                           [=](int z, int y) {
-                               float *r = ph + (z * Y + y) * X;
-                               return [=](int x, float v) { r[x] = v; };
-                           });
+        mmsconv::rows_back<mmsconv::row_pairs<decltype(pl)>(CONV_THREADS, CONV_PAIRS)>(
+            pl, c, cbuf, it.first, min(c.fb, np), [=](int k) { return st + k * cs; },
+            [=](int z, int y) {
+                float *r = ph + (z * Y + y) * X;
+                return [=](int x, float v) { r[x] = v; };
+            });
     });
 }
 

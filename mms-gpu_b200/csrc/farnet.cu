@@ -9,14 +9,16 @@
 // (levels 2..L, level-major, box row-major inside a level):
 //   M   multipoles           Lf  final locals (M2L + L2L of the parent's)
 //   dM  dloss/dM             dL  dloss/dLf
-// Every forward and adjoint kernel gives each output element to one thread
-// (no atomics: fixed summation order, reproducible bits): the levels that do
-// not depend on one another share a launch (the interaction lists of every
-// level), the chains along the tree are a CTA per level-2 box that walks its
-// levels.  The gradients of the translation tables are sums of outer products
+// Every forward and adjoint kernel gives each output element to one thread (no
+// atomics: fixed summation order, reproducible bits, of the gradients too; the
+// loss alone is added up over CTAs by FP64 atomics, so its last bits vary): the
+// levels that do not depend on one another share a launch (the interaction lists
+// of every level), the chains along the tree are a CTA per level-2 box that walks
+// its levels.  The gradients of the translation tables are sums of outer products
 // over boxes and samples with 320 wanted entries an operator, in FP32 registers
 // (k_t_opgrad; within 5e-6 of the split-BF16 GEMMs they were); those of the
-// encoder and the decoder, 192 x 24 with K = boxes x samples, are GEMMs: the operands are gathered into K-major BF16 hi/lo planes
+// encoder and the decoder, 192 x 24 with K = boxes x samples, are GEMMs: the
+// operands are gathered into K-major BF16 hi/lo planes
 // ([hi | lo | hi] against [hi | hi | lo], relative error ~2^-16 per product)
 // and multiplied by the tcgen05 core (umma_gemm_bf16_splitk: the long K range
 // split over CTAs, the partials summed in a fixed order).
@@ -772,7 +774,9 @@ OpK opk(const mms_farnet *n, int nbatch)
 {
     OpK k{};
     int at = 0;
-    // about 64 boxes a thread, whole lines of a level
+    // 32 boxes a thread or more, whole lines of a level; from 24 chunks on (768
+    // boxes of a class) the chunks get longer with the batch: 8 x 256 x 256 85
+    // boxes, an FP32 sum of as many products
     auto chunks = [](long long boxes, long long lines) {
         return (int)std::max(1LL, std::min({(long long)OP_MAX_CHUNKS, boxes / 32, lines}));
     };
@@ -781,7 +785,8 @@ OpK opk(const mms_farnet *n, int nbatch)
         k.m2l_ch[l] = chunks((long long)nbatch << (2 * (l - 1)), (long long)nbatch << (l - 1));
         at += 4 * k.m2l_ch[l];
     }
-    for (int l = 2; l < n->L; l++) k.par_ch[l] = chunks(((long long)nbatch << (2 * l)) / OP_SUB, ((long long)nbatch << l) / OP_SUB);
+    for (int l = 2; l < n->L; l++)
+        k.par_ch[l] = chunks(((long long)nbatch << (2 * l)) / OP_SUB, ((long long)nbatch << l) / OP_SUB);
     k.m2m[2] = at;
     for (int l = 2; l < n->L; l++) {
         k.m2m[l] = at;

@@ -2396,7 +2396,9 @@ int fmm_set_carveout()
                        (const void *)k_top_m2m,    (const void *)k_top_l2l,     (const void *)k_l2l_c,
                        (const void *)k_m2l_split,  (const void *)k_m2l_gather,  (const void *)k_m2l_gemm};
     for (const void *fn : k) MMS_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, c));
-#define X(a, b) MMS_CUDA_TRY(cudaFuncSetAttribute(k_m2l_res<a, b, 16>, cudaFuncAttributePreferredSharedMemoryCarveout, c)); MMS_CUDA_TRY(cudaFuncSetAttribute(k_m2l_res<a, b, 32>, cudaFuncAttributePreferredSharedMemoryCarveout, c));
+#define X(a, b)                                                                                               \
+    MMS_CUDA_TRY(cudaFuncSetAttribute(k_m2l_res<a, b, 16>, cudaFuncAttributePreferredSharedMemoryCarveout, c)); \
+    MMS_CUDA_TRY(cudaFuncSetAttribute(k_m2l_res<a, b, 32>, cudaFuncAttributePreferredSharedMemoryCarveout, c));
     MMS_M2L_RES_CASES(X)
 #undef X
 #define X(S_, B_)                                                                                            \
@@ -2943,10 +2945,10 @@ static int l2p_wide_launch(const FmmPlan *pl, const float *near, const float *Lg
                          (size_t)f.NR * (NB + 1 + NP + GX)) * sizeof(float);
     // a warp a layer; more of them, for the locals alone, where those are many
     // (400 x 400 x 2, leaf 4, P = 8: 424 -> 370 us a potential)
-    MMS_CUDA_TRY(launch_k(k_l2p_wide<S, R>, dim3(div_up(f.X, 32), div_up(f.Y, R * S)),
-                          dim3(std::max(32 * f.Z, std::min(256, (NB * f.NR / 16 + 31) / 32 * 32))), smem, st, near, (const float *)(pl->Lpart + pl->lev_off[f.L] * f.NR),
-                          (const float *)pl->Tl2l, (const float *)pl->Vt, phi, f, pl->nbox_total * f.NR, nsplit, Lgp, Lpp,
-                          nnear, near_stride));
+    const int threads = std::max(32 * f.Z, std::min(256, (NB * f.NR / 16 + 31) / 32 * 32));
+    MMS_CUDA_TRY(launch_k(k_l2p_wide<S, R>, dim3(div_up(f.X, 32), div_up(f.Y, R * S)), dim3(threads), smem, st, near,
+                          (const float *)(pl->Lpart + pl->lev_off[f.L] * f.NR), (const float *)pl->Tl2l,
+                          (const float *)pl->Vt, phi, f, pl->nbox_total * f.NR, nsplit, Lgp, Lpp, nnear, near_stride));
     return MMS_OK;
 }
 

@@ -117,8 +117,10 @@ class Ensemble:
         _check(load().mms_ens_sync(self.h))
 
     def autotune(self, reps=5):
-        """measured shape of the batched direct kernel: (warps per CTA, source
-        rows per batch, ms per potential)"""
+        """measured shape of the batched pair sum: (warps per CTA, source rows
+        per batch, ms per potential).  Where the potential is a convolution there is
+        no shape to choose: the first two are those of the pair sum it does not
+        run, the third is the time of one potential"""
         w, q, ms = ctypes.c_int(), ctypes.c_int(), ctypes.c_double()
         _check(load().mms_ens_autotune(self.h, reps, ctypes.byref(w), ctypes.byref(q), ctypes.byref(ms)))
         return w.value, q.value, ms.value

@@ -99,3 +99,28 @@ def test_small_grids_in_one_launch(cuda, lib, oracle_mod, dims):
     assert np.linalg.norm(phi.cpu().numpy() - ref) <= 2e-6 * np.linalg.norm(ref)
     Mo = oracle_mod.rk4_run(og, oracle_mod.Params(), np.ones((Z, Y, X), np.uint8), M, 1e-13, 1)
     assert max_angle_deg(M1, Mo) < 1e-4
+
+
+# the column CTAs hold all layers of a column in 200 KB of shared memory: on both
+# sides of that limit, the second of each pair takes the pair sum
+@pytest.mark.parametrize("dims,conv", [((3, 1024, 3), True), ((3, 1025, 3), False), ((3, 768, 6), True),
+                                       ((3, 769, 6), False), ((3, 512, 8), True), ((3, 513, 8), False),
+                                       ((1025, 3, 3), True), ((71, 9, 8), True), ((71, 8, 9), False)])
+def test_grids_at_the_column_limit(cuda, lib, oracle_mod, dims, conv):
+    """the convolution's tolerance where it serves, else the pair sum's (2e-6)"""
+    import mmsb200
+    torch = cuda
+    d = (5e-9, 4e-9, 6e-9)
+    X, Y, Z = dims
+    rho_h = (np.random.default_rng(X + 31 * Y + Z).standard_normal((Z, Y, X)) * 1e14).astype(np.float32)
+    rho = torch.from_numpy(rho_h).cuda()
+    phi = torch.full_like(rho, float("nan"))
+    with mmsb200.Context(mmsb200.Grid(X, Y, Z, *d)) as ctx:
+        ctx.potential_dev(rho, phi)
+        ctx.sync()
+        before = ctx.kernel_launches
+        ctx.potential_dev(rho, phi)
+        assert ctx.kernel_launches - before == (3 if conv else 1)
+        ctx.sync()
+    ref = oracle_mod.potential_direct(oracle_mod.Grid(X, Y, Z, *d), rho_h.astype(np.float64))
+    assert rel_l2(phi.cpu().numpy(), ref) <= (6.1e-8 if conv else 2e-6)
