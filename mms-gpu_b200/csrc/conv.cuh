@@ -52,8 +52,9 @@ struct Radices {
 // The lengths, in two sets of radices.  Single grids take small ones: many
 // threads with little each, so that a launch of a few CTAs ends soon (64 x 64 x 3:
 // 77 us a step against 89 with the other set).  Batches take few passes with
-// balanced radices, and stop at 512 (512 instances: 602 us a step against 710).
-constexpr int NPLANS = 19, NBATCH = 13;
+// balanced radices, at most 64 butterflies each (the threads of their CTAs; none for
+// 384), and stop at 512 (512 instances: 602 us a step against 710).
+constexpr int NPLANS = 19, NBATCH = 12;
 template <class F>
 void with_plan(int id, F &&f)
 {
@@ -92,8 +93,7 @@ void with_plan(int id, F &&f)
     case 8: f(Radices<8, 8, 3>{}); break;                    \
     case 9: f(Radices<8, 8, 4>{}); break;                    \
     case 10: f(Radices<8, 8, 5>{}); break;                   \
-    case 11: f(Radices<16, 8, 3>{}); break;                  \
-    case 12: f(Radices<8, 8, 8>{}); break;
+    case 11: f(Radices<8, 8, 8>{}); break;
 
 template <class F>
 void with_batch_plan_host(int id, F &&f)
