@@ -71,8 +71,10 @@ __global__ void k_conv_table_y(const double *__restrict__ T, double *__restrict_
 
 // ---- the passes with the columns in device memory [kx][z][y] -------------------
 // Three launches a potential.  Up to about 200 cells a side they are bound by
-// launch and barrier latency (4 us each), beyond by the column store's traffic
-// through L2 (32 bytes a cell and pass) and the FP64 passes.  Measured, whole
+// launch and barrier latency (4 us each); at 256 x 256 x 3 still by the latency of
+// loads (8 to 11 warps an SM, issue 13 to 18 %, FP64 pipe 8 to 14 %, L2 6 %).
+// Beyond, the column store's traffic grows with the cells (32 bytes a cell and
+// pass).  Measured, whole
 // potential, against the pair sum: 64 x 64 x 3 8.7 us (100 us), 256 x 256 x 3
 // 18.7 us (2,056 us), 512 x 512 x 3 68 us (23.9 ms), 1024 x 1024 x 3 294 us
 // (382 ms); rel-L2 against the FP64 sum 2.5e-8 at every size, the rounding of

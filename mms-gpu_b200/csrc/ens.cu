@@ -198,8 +198,8 @@ __global__ void __launch_bounds__(ETPB) k_ens_stage(const float *__restrict__ ph
 // CTAs run the same code.  512 instances of 16 .. 64 x 16 .. 64 x 3 (2.34 M
 // cells): 120 us a potential (rows 46, columns 69, back 22 us cold) against
 // 770 us for the pair sum, 602 us a step against 3,973.  Bound by the latency of
-// the passes: 14 to 20 warps an SM at 92 to 128 registers, issue 23 to 31 %,
-// FP64 pipe 9 to 22 %, L2 20 %.  A cluster of CTAs per instance with the
+// the passes: 15 to 19 warps an SM at 94 to 128 registers, issue 24 to 31 %,
+// FP64 pipe 10 to 22 %, L2 8 to 21 %.  A cluster of CTAs per instance with the
 // columns in distributed shared memory (a whole step in one launch) took 767
 // us a step: its few warps work through long instruction streams alone.
 constexpr int CONV_THREADS = 64;  // 128: 936 us a step of 512 instances against 782

@@ -28,8 +28,8 @@
 // GEMM (a 58 MB operand for the leaf level's interaction lists): some 75
 // launches, the largest 138, 130 and 128 us.  Now 278 us: 19 launches of 205 us
 // (lists 2 x 22, k_t_opgrad 24, leaves 17, operands 17, GEMMs and their sums
-// 39, chains 35), bound by issue with few warps and by latency, and the results'
-// way to the host.
+// 39, chains 35), bound by latency with few warps an SM (the lists by shared-memory
+// reads), and the results' way to the host.
 #include <math.h>
 #include <string.h>
 
@@ -304,7 +304,7 @@ __device__ __forceinline__ void fma2(float2 &acc, float2 a, float2 b)
 // every lane multiplies its row by the operator's, read as 16-byte broadcasts.
 //   forward: out[t] = sum_o T[o] in[t - o], o in the list of t
 //   ADJ:     out[s] = sum_o T[o]^T in[s + o], o in the list of s + o
-// Bound by instruction issue with few warps a scheduler.  8 x 256 x 256: 27 us
+// Bound by shared-memory reads (L1 pipe 70 %, issue 33 %).  8 x 256 x 256: 27 us
 // with a third of the channels a warp and rows of its own, 34 us with two
 // boxes a lane besides (half the operator reads, half the warps); 22 us as here.
 constexpr int LAT_BOXES = 32, LAT_THREADS = 6 * 32;
