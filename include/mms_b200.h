@@ -52,7 +52,12 @@ typedef enum {
 } mms_status;
 
 typedef enum {
-    MMS_SOLVER_DIRECT = 0,   /* exact O(N^2) sum, FP32 tiles, compensated      */
+    MMS_SOLVER_DIRECT = 0,   /* exact sum: an FP64 convolution, or one launch of
+                                FP32 row sums for small grids; grids without a
+                                transform plan (more than 8 layers; with ydim
+                                beyond 512, 768, 1024 more than 7, 5, 2; no
+                                memory for it) take the O(N^2) pair sum, FP32
+                                tiles, compensated                            */
     MMS_SOLVER_FMM = 1,      /* spherical-harmonic FMM, exact near field       */
     MMS_SOLVER_SURROGATE = 2 /* exact near field (FMM P2P, leaf 8) + far field
                                 from the learned operator (mms_farnet_*); the
